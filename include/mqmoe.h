@@ -259,6 +259,17 @@ int mq_w4a16_grouped_swiglu(const void* x,
                             int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H, int64_t group_size,
                             void* h, void* stream);
 
+/* mq_w4a16_grouped_swiglu on rows gathered inside the kernel: row p of the expert-sorted order is x[perm[p] / top_k]
+ * of the unpermuted x [T,H] (what mq_permute_plan lists; replaces the row gather of
+ * mini_qwen/kernels/moe_permute.py:30 in front of the expert loop of mini_qwen/model/layers/moe.py:59-65).
+ * For prefill-size groups: group_size == 128, H % 128 == 0, I % 32 == 0, E <= 1024; the tensors 16-byte aligned. */
+int mq_w4a16_grouped_swiglu_gather(const void* x, const int32_t* perm,
+                                   const int32_t* qweight_gate, const void* scales_gate, const int32_t* qzeros_gate,
+                                   const int32_t* qweight_up, const void* scales_up, const int32_t* qzeros_up,
+                                   const int32_t* offsets, int64_t T, int64_t top_k, int64_t E,
+                                   int64_t weight_period, int64_t I, int64_t H, int64_t group_size,
+                                   void* h, int32_t* d_status, void* stream);
+
 /* The same two operations with PREPARED activations, the form the block's decode path uses (same results as
  * the two calls above up to the order of the fp32 sums):
  *   xp [S,Kd] (16-bit): the expert-sorted rows.  x_format 0: bf16, natural k order.  1: bf16 with the k order

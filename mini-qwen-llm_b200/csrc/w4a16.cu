@@ -24,8 +24,6 @@
 //   * Every lane moves its own 16-byte pieces (weights and activations) through an 8-deep ring of
 //     cp.async copies in shared memory: a lane only reads what it copied itself, so the ring needs
 //     no barrier and has no bank conflicts, and 12 KB per warp are in flight while it computes.
-#include <cstdlib>
-
 #include "common.cuh"
 
 namespace mq {
@@ -387,6 +385,13 @@ int w4a16_stream(const void* x, const float* xs, int x_format, const int32_t* pe
                  const int32_t* qz1, bool swiglu, bool shuffle_out, const int32_t* offsets, int64_t S, int64_t E,
                  int64_t period, int64_t N, int64_t Kd, void* out, int32_t* d_status, cudaStream_t st);
 
+// Tensor-core tile kernel for prefill-size groups (w4a16_tile.cu).
+bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
+int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k, const int32_t* qw0, const void* sc0,
+               const int32_t* qz0, const int32_t* qw1, const void* sc1, const int32_t* qz1, bool swiglu,
+               const int32_t* offsets, int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, void* out,
+               int32_t* d_status, cudaStream_t st);
+
 namespace {
 
 int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* offsets, int64_t S, int64_t E,
@@ -401,10 +406,17 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
   if (swiglu && (!p1.qw || !p1.sc || !p1.qz)) return MQ_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(p0.qw) || !aligned16(p0.sc) || !aligned16(out)) return MQ_ERR_INVALID_ARGUMENT;
   if (swiglu && (!aligned16(p1.qw) || !aligned16(p1.sc))) return MQ_ERR_INVALID_ARGUMENT;
-  // Which kernel: the TMA-staged stream kernel is the faster one for the fused gate/up projection from a few
-  // dozen slots on (batch 64: 66 against 81 us; below 32 slots both are bound by launch latency), the per-lane
-  // cp.async kernel below for the single projection (40 against 43 us at batch 64: its K is short and it needs
-  // no K split).  The prepared-activation entry points ask for the stream kernel explicitly.
+  // Which kernel.  More than one block of eight rows per group on average: the tensor-core tile kernel, which
+  // unpacks a weight once for up to 128 rows (gate/up of the 128-expert layer, cold: 94 against 106 us at 128 tokens,
+  // 125 against 107 at 192; a 2048 x 4096 linear: 12.4 against 17.4 us at 8 rows, 17.4 against 17.4 at 9, 115 against
+  // 18 at 64).  Below that the TMA-staged stream kernel is the faster one for the fused gate/up projection from a few
+  // dozen slots on (below 32 slots both are bound by launch latency), the per-lane cp.async kernel for the single
+  // projection (its K is short and it needs no K split).  The prepared-activation entry points ask for the stream
+  // kernel explicitly.
+  if (!want_stream && x_format == 0 && S > 8 * E && w4a16_tile_covers(S, E, period, N, Kd, group) && aligned16(p0.qz) &&
+      (!swiglu || aligned16(p1.qz)) && S * (Kd / 8) < ((int64_t)1 << 32))
+    return w4a16_tile(x, S, nullptr, 1, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, offsets, S, E, period, N, Kd,
+                      out, d_status, st);
   const bool stream = want_stream || (swiglu && S >= 32);
   if (stream && w4a16_stream_covers(S, E, period, N, Kd, group))
     return w4a16_stream(x, xs, x_format, perm, top_k, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, shuffle_out,
@@ -446,6 +458,26 @@ extern "C" int mq_w4a16_grouped_swiglu(const void* x,
   mq::W4Proj pu{qweight_up, reinterpret_cast<const __nv_bfloat16*>(scales_up), qzeros_up};
   return mq::launch_w4(x, pg, pu, true, offsets, S, E, weight_period, I, H, group_size, h,
                        reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mq_w4a16_grouped_swiglu_gather(const void* x, const int32_t* perm,
+                                              const int32_t* qweight_gate, const void* scales_gate,
+                                              const int32_t* qzeros_gate, const int32_t* qweight_up,
+                                              const void* scales_up, const int32_t* qzeros_up, const int32_t* offsets,
+                                              int64_t T, int64_t top_k, int64_t E, int64_t weight_period, int64_t I,
+                                              int64_t H, int64_t group_size, void* h, int32_t* d_status, void* stream) {
+  using namespace mq;
+  if (T < 0 || top_k <= 0 || E <= 0 || I <= 0 || H <= 0 || group_size <= 0 || weight_period <= 0 || weight_period > E)
+    return MQ_ERR_INVALID_ARGUMENT;
+  const int64_t S = T * top_k;
+  if (!w4a16_tile_covers(S, E, weight_period, I, H, group_size)) return MQ_ERR_UNSUPPORTED_SHAPE;
+  if (S == 0) return MQ_OK;
+  for (const void* p : {x, scales_gate, scales_up, (const void*)qweight_gate, (const void*)qweight_up,
+                        (const void*)qzeros_gate, (const void*)qzeros_up, (const void*)h})
+    if (p == nullptr || !aligned16(p)) return MQ_ERR_INVALID_ARGUMENT;
+  if (!perm || !offsets) return MQ_ERR_INVALID_ARGUMENT;
+  return w4a16_tile(x, T, perm, top_k, qweight_gate, scales_gate, qzeros_gate, qweight_up, scales_up, qzeros_up, true,
+                    offsets, S, E, weight_period, I, H, h, d_status, reinterpret_cast<cudaStream_t>(stream));
 }
 
 /* Prepared-activation forms: see include/mqmoe.h. */

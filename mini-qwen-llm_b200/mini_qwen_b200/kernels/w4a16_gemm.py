@@ -85,6 +85,34 @@ def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zer
     return h
 
 
+def w4a16_gather_supported(hidden: int, out_features: int, group_size: int, groups: int) -> bool:
+    """Shapes :func:`w4a16_grouped_swiglu_gather` covers."""
+    return group_size == 128 and hidden % 128 == 0 and out_features % 32 == 0 and groups <= 1024
+
+
+def w4a16_grouped_swiglu_gather(x, perm, top_k: int, gate, up, expert_offsets, group_size: int = 128,
+                                status: torch.Tensor | None = None) -> torch.Tensor:
+    """:func:`w4a16_grouped_swiglu` on ``x[perm // top_k]`` without materialising the permuted rows (the tensor-core
+    kernel for prefill-size groups gathers them itself).  ``x`` is the unpermuted [T, H]."""
+    E = gate[0].shape[0]
+    K, N = _check_w4(x, *gate, group_size, E)
+    _check_w4(x, *up, group_size, E)
+    expert_offsets = _offsets32(expert_offsets)
+    groups = expert_offsets.numel() - 1
+    assert groups >= E and groups % E == 0 and perm.dtype == torch.int32 and perm.is_contiguous()
+    x = x.contiguous()
+    T, S = x.shape[0], perm.numel()
+    assert S == T * top_k
+    h = torch.empty(S, N, dtype=torch.bfloat16, device=x.device)
+    rc = _cabi.load().mq_w4a16_grouped_swiglu_gather(
+        _cabi.ptr(x), _cabi.ptr(perm), _cabi.ptr(gate[0]), _cabi.ptr(gate[1]), _cabi.ptr(gate[2]), _cabi.ptr(up[0]),
+        _cabi.ptr(up[1]), _cabi.ptr(up[2]), _cabi.ptr(expert_offsets), T, top_k, groups, E, N, K, group_size,
+        _cabi.ptr(h), _cabi.ptr(status), _cabi.stream_ptr(x.device))
+    _cabi.check(rc, "mq_w4a16_grouped_swiglu_gather")
+    _cabi.count_launches(1 if S else 0)
+    return h
+
+
 def w4a16_gemm(
     x: torch.Tensor,
     qweight: torch.Tensor,

@@ -1,0 +1,82 @@
+"""The W4A16 tile kernel for prefill-size groups (csrc/w4a16_tile.cu): single linears and grouped projections at the
+edges of its tiles (rows 9 to 129 around the 16-row steps and the 128-row tile, columns that end inside a tile or after
+the first of a pair, one and several quantisation groups, empty experts), with contiguous and with gathered rows.
+
+Single linears are held to the fp32 result of the oracle's formula: the kernel multiplies exact integers q - z and adds
+fp32 sums, so only the summation order (about 2^-22 of the sum of magnitudes) and the final rounding to bf16 (2^-9
+relative) can differ.  The grouped projections are held to cases.w4_output_bar."""
+import pytest
+import torch
+
+import cases
+from mini_qwen_b200 import _cabi, synthetic
+from mini_qwen_b200.kernels import moe_permute_plan
+from mini_qwen_b200.kernels.moe_permute import gather_rows
+from mini_qwen_b200.kernels.w4a16_gemm import (w4a16_gemm, w4a16_grouped_gemm, w4a16_grouped_swiglu,
+                                               w4a16_grouped_swiglu_gather)
+from oracle import moe_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda", 0)
+
+
+@pytest.mark.parametrize("M,K,N", [(9, 128, 32), (16, 256, 128), (17, 384, 96), (127, 128, 160), (128, 512, 256),
+                                   (129, 256, 384), (300, 128, 4096), (2500, 256, 640)])
+def test_single_linear_at_the_edges_of_the_tiles(M, K, N):
+    g = torch.Generator().manual_seed(M + K + N)
+    w = torch.randn(K, N, generator=g) * 0.05
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    qw, sc, qz = O.minmax_quantize(w, 128)
+    got = w4a16_gemm(x.to(DEV), qw.contiguous().to(DEV), sc.to(DEV), qz.to(DEV), 128).cpu().double()
+    ref = O.w4a16_linear(x, qw, sc, qz, 128, torch.float64).double()      # exact sums, rounded to bf16
+    q = torch.stack([(qw >> (4 * i)) & 15 for i in range(8)], 1).reshape(K, N).double()
+    z = torch.stack([(qz >> (4 * i)) & 15 for i in range(8)], 2).reshape(K // 128, N).double()
+    dq = (q - z.repeat_interleave(128, 0)) * sc.double().repeat_interleave(128, 0)
+    terms = x.double().abs() @ dq.abs()                                    # sum of magnitudes
+    # one bf16 step (two roundings of neighbouring fp32 values may fall apart by one) and the fp32 summation error
+    bound = 2.0 ** -7 * ref.abs() + 2.0 ** -20 * terms
+    assert bool(((got - ref).abs() <= bound).all())
+
+
+def dev_set(p):
+    return tuple(t.to(DEV) for t in (p.qweight, p.scales.to(torch.bfloat16), p.qzeros))
+
+
+@pytest.mark.parametrize("T,H,E,K,I,hot", [(37, 128, 4, 2, 32, 0), (65, 256, 4, 2, 160, 0), (200, 256, 8, 4, 384, 2),
+                                           (300, 640, 6, 2, 128, 1)])
+def test_grouped_projections_match_the_oracle(T, H, E, K, I, hot):
+    """``hot`` experts take every token (groups of several tiles) and the last expert none."""
+    lay = synthetic.w4a16_layer(T + I, T, H, E, K, I, group=128) if I % 128 == 0 else None
+    g = torch.Generator().manual_seed(T)
+    if lay is None:        # I that is no multiple of the quantisation group: gate/up only
+        gate, up = synthetic._w4_proj(g, E, H, I, 128), synthetic._w4_proj(g, E, H, I, 128)
+        x, down = torch.randn(T, H, generator=g).to(torch.bfloat16), None
+    else:
+        gate, up, down, x = lay.gate, lay.up, lay.down, lay.x
+    ids = torch.stack([torch.cat([torch.arange(hot), hot + torch.randperm(E - 1 - hot, generator=g)[:K - hot]])
+                       for _ in range(T)]).to(torch.int32).to(DEV)
+    perm, _, off32, _ = moe_permute_plan(ids, E, want_int64_offsets=False)
+    xd = x.to(DEV)
+    rows = gather_rows(xd, perm, K)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    h = w4a16_grouped_swiglu_gather(xd, perm, K, dev_set(gate), dev_set(up), off32, status=status)
+    assert torch.equal(w4a16_grouped_swiglu(rows, dev_set(gate), dev_set(up), off32), h)
+    off, sets = off32.cpu(), tuple((p.qweight, p.scales.to(torch.bfloat16), p.qzeros) for p in (gate, up))
+    h32, h64 = (cases.w4_grouped_reference(rows.cpu(), sets, off, t) for t in (torch.float32, torch.float64))
+    cases.w4_output_bar(h.cpu(), h32, h64)
+    if down is not None:
+        o = w4a16_grouped_gemm(h, *dev_set(down), off32)
+        dset = ((down.qweight, down.scales.to(torch.bfloat16), down.qzeros),)
+        o32, o64 = (cases.w4_grouped_reference(h.cpu(), dset, off, t) for t in (torch.float32, torch.float64))
+        cases.w4_output_bar(o.cpu(), o32, o64)
+    assert status.item() == 0
+
+
+def test_gather_entry_point_rejects_what_the_kernel_does_not_cover():
+    x = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
+    w = tuple(t.to(DEV) for t in (torch.zeros(1, 16, 40, dtype=torch.int32), torch.zeros(1, 1, 40, dtype=torch.bfloat16),
+                                  torch.zeros(1, 1, 5, dtype=torch.int32)))
+    perm = torch.arange(4, dtype=torch.int32, device=DEV)
+    off = torch.tensor([0, 4], dtype=torch.int32, device=DEV)
+    with pytest.raises(ValueError):
+        w4a16_grouped_swiglu_gather(x, perm, 1, w, w, off)                 # 40 columns: not a multiple of 32
