@@ -252,6 +252,10 @@ int mq_w4a16_grouped_gemm(const void* x, const int32_t* qweight, const void* sca
 
 /* Fused W4A16 gate/up projection with SwiGLU (bf16 rounding after gate, silu, up and the
  * product, as LinearW4A16 returns bf16).  Both projections share shapes: Kd = H, N = I. */
+/* One linear (LinearW4A16.forward, mini_qwen/model/layers/linear_w4a16.py:31-36): mq_w4a16_grouped_gemm with a single
+ * group of M rows, without an offsets array. */
+int mq_w4a16_linear(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros, int64_t M,
+                    int64_t N, int64_t Kd, int64_t group_size, void* out, void* stream);
 int mq_w4a16_grouped_swiglu(const void* x,
                             const int32_t* qweight_gate, const void* scales_gate, const int32_t* qzeros_gate,
                             const int32_t* qweight_up, const void* scales_up, const int32_t* qzeros_up,
@@ -324,6 +328,32 @@ int mq_w4a16_tc_swiglu(const void* xp, const float* xs,
                        const int32_t* qweight_up, const void* scales_up, const int32_t* qzeros_up,
                        const int32_t* offsets, int64_t S, int64_t E, int64_t weight_period, int64_t I,
                        int64_t H, int64_t group_size, void* h_shuffled, int32_t* d_status, void* stream);
+
+/* ------------------------------------------------------------------------------------------
+ * The whole block in one call: what Qwen3MoEBlock.forward (mini_qwen/model/layers/moe.py:49-68) computes on one
+ * GPU, as the chain of the calls above with every intermediate in one caller workspace.  norm_weight != NULL puts
+ * the decoder layer's RMSNorm in front, residual != NULL its add behind (mini_qwen/model/qwen3_moe.py:63-66);
+ * residual and out are [T, hidden] of L->dtype, as x is.
+ *   dense layers (group_size 0, any dtype): gate[0] = w13 [E, 2*inter, hidden] (gate rows, then up rows),
+ *     down[0] = w2 [E, hidden, inter];
+ *   W4A16 layers (dtype MQ_BF16): gate / up / down = {qweight, scales, qzeros} of the stacks.
+ * route_workspace: as mq_route_small's (zero-filled once by the caller, for 64 tokens, kept between calls that are
+ * ordered with one another); read for T <= 64 only.  workspace: mq_moe_forward_workspace_bytes(layer, T) bytes,
+ * overwritten.  h_launches (optional) receives the number of kernels launched. */
+typedef struct {
+  int64_t hidden, inter, experts, top_k, group_size;
+  int32_t dtype, router_dtype, renormalize, reserved;
+  const void* router;            /* [experts, hidden] */
+  const float* router_bias;      /* [experts] or NULL */
+  const void* gate[3];
+  const void* up[3];
+  const void* down[3];
+} mq_moe_layer;
+size_t mq_moe_forward_workspace_bytes(const mq_moe_layer* h_layer, int64_t T);
+int mq_moe_forward(const mq_moe_layer* h_layer, const void* x, const void* norm_weight, float norm_eps,
+                   const void* residual, int64_t T, void* route_workspace, size_t route_workspace_bytes,
+                   void* workspace, size_t workspace_bytes, void* out, int32_t* d_status,
+                   int32_t* h_launches, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Expert parallelism over peer memory (no counterpart in the reference, which is single-GPU).

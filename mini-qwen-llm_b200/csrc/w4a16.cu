@@ -174,7 +174,7 @@ __device__ int nth_nonempty(const int32_t* offsets, int E, int y, int* s_e) {
 template <bool SWIGLU, int KSPLIT>
 __global__ void __launch_bounds__(W4_WARPS * 32, 4)
 w4a16_grouped_kernel(const __nv_bfloat16* __restrict__ x, W4Proj p0, W4Proj p1,
-                     const int32_t* __restrict__ offsets, int E, int period, int N, int Kd, int group,
+                     const int32_t* __restrict__ offsets, int S, int E, int period, int N, int Kd, int group,
                      int compact, __nv_bfloat16* __restrict__ out) {
   // SWIGLU: the two streams of a warp are the gate and up projections of the same 32 columns.
   // Plain: the two streams are adjacent 32-column tiles (64 columns per warp).
@@ -190,8 +190,8 @@ w4a16_grouped_kernel(const __nv_bfloat16* __restrict__ x, W4Proj p0, W4Proj p1,
     __syncthreads();                     // everyone has read it before any copy lands in the ring
   }
   if (e < 0) return;
-  const int row_lo = offsets[e];
-  const int rows = offsets[e + 1] - row_lo;
+  const int row_lo = offsets != nullptr ? offsets[e] : 0;        // no offsets: one group of all S rows
+  const int rows = offsets != nullptr ? offsets[e + 1] - row_lo : S;
   if (rows <= 0) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -372,7 +372,7 @@ void launch_w4_variant(const void* x, W4Proj p0, W4Proj p1, const int32_t* offse
   const int compact = S < E;
   dim3 grid((unsigned)((N + cols_per_cta - 1) / cols_per_cta), (unsigned)(compact ? S : E));
   launch_after_predecessor(w4a16_grouped_kernel<SWIGLU, KSPLIT>, grid, dim3(W4_WARPS * 32), 0, st,
-                           reinterpret_cast<const __nv_bfloat16*>(x), p0, p1, offsets, (int)E, (int)period, (int)N,
+                           reinterpret_cast<const __nv_bfloat16*>(x), p0, p1, offsets, (int)S, (int)E, (int)period, (int)N,
                            (int)Kd, (int)group, compact, reinterpret_cast<__nv_bfloat16*>(out));
 }
 
@@ -402,7 +402,8 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
   if (period <= 0 || period > E) return MQ_ERR_INVALID_ARGUMENT;
   if (group % 32 != 0 || Kd % group != 0 || N % 8 != 0 || E > 65535) return MQ_ERR_UNSUPPORTED_SHAPE;
   if (S == 0) return MQ_OK;
-  if (!x || !p0.qw || !p0.sc || !p0.qz || !offsets || !out) return MQ_ERR_INVALID_ARGUMENT;
+  if (!x || !p0.qw || !p0.sc || !p0.qz || !out) return MQ_ERR_INVALID_ARGUMENT;
+  if (!offsets && (E != 1 || want_stream || swiglu)) return MQ_ERR_INVALID_ARGUMENT;
   if (swiglu && (!p1.qw || !p1.sc || !p1.qz)) return MQ_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(p0.qw) || !aligned16(p0.sc) || !aligned16(out)) return MQ_ERR_INVALID_ARGUMENT;
   if (swiglu && (!aligned16(p1.qw) || !aligned16(p1.sc))) return MQ_ERR_INVALID_ARGUMENT;
@@ -446,6 +447,12 @@ extern "C" int mq_w4a16_grouped_gemm(const void* x, const int32_t* qweight, cons
   mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
   return mq::launch_w4(x, p, p, false, offsets, S, E, weight_period, N, Kd, group_size, out,
                        reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mq_w4a16_linear(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros, int64_t M,
+                               int64_t N, int64_t Kd, int64_t group_size, void* out, void* stream) {
+  mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
+  return mq::launch_w4(x, p, p, false, nullptr, M, 1, 1, N, Kd, group_size, out, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mq_w4a16_grouped_swiglu(const void* x,

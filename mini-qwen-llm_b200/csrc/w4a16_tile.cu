@@ -58,7 +58,8 @@ struct TileParams {
   const __nv_bfloat16* x;                        // token rows [*, Kd]
   const int32_t* perm;                           // optional: sorted row p is x[perm[p] / top_k]
   int top_k;
-  const int32_t* offsets;                        // [E + 1]
+  const int32_t* offsets;                        // [E + 1], or null: one group of all S rows
+  int S;
   int E, period, N, Kd, tn;                      // tn: most tokens per tile (a multiple of 16)
   TileProj p0, p1;
   __nv_bfloat16* out;                            // [*, N]
@@ -137,7 +138,7 @@ w4a16_tile_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_const
     mbar_init_fence();
   }
   if (warp == 1) tmem_alloc(smem_addr((const void*)tmem_ptr), 512u);
-  for (int e = threadIdx.x; e <= E; e += TL_THREADS) s_off[e] = P.offsets[e];
+  for (int e = threadIdx.x; e <= E; e += TL_THREADS) s_off[e] = P.offsets != nullptr ? P.offsets[e] : e * P.S;
   __syncthreads();
   if (warp == 0) {                                              // first[]: exclusive sums of the groups' tile counts
     int carry = 0;
@@ -527,6 +528,7 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
   P.perm = perm;
   P.top_k = (int)top_k;
   P.offsets = offsets;
+  P.S = (int)S;
   P.E = (int)E;
   P.period = (int)period;
   P.N = (int)N;

@@ -40,6 +40,7 @@ PROTOTYPES = {
     "mq_grouped_swiglu_gather": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _I, _P, _P, _P]),
     "mq_stack_tensors": (c_int, [_P, _L, _L, _I, _P, _P]),
     "mq_w4a16_grouped_gemm": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
+    "mq_w4a16_linear": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_grouped_swiglu": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_grouped_swiglu_gather": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_stream_swiglu": (c_int, [_P, _P, _I, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _I, _P, _P, _P]),
@@ -47,6 +48,8 @@ PROTOTYPES = {
     "mq_w4a16_tc_prep": (c_int, [_P, _P, _L, _L, _L, _I, _P, _P, _P]),
     "mq_w4a16_tc_gemm": (c_int, [_P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_tc_swiglu": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
+    "mq_moe_forward_workspace_bytes": (c_size_t, [_P, _L]),
+    "mq_moe_forward": (c_int, [_P, _P, _P, c_float, _P, _L, _P, c_size_t, _P, c_size_t, _P, _P, _P, _P]),
     "mq_ep_share_counts": (c_int, [_P, _L, _L, _L, _P, _P]),
     "mq_ep_barrier": (c_int, [_P, _P, _L, _L, _L, _P, _P]),
     "mq_ep_plan": (c_int, [_P, _L, _L, _L, _P, _P, _P]),
@@ -59,6 +62,14 @@ PROTOTYPES = {
     "mq_ep_send_partials": (c_int, [_P, _I, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P, _P, _L, _P, _P]),
     "mq_ep_sum_partials": (c_int, [_P, _I, _P, _L, _L, _L, _P, _P]),
 }
+
+class MoELayer(ctypes.Structure):
+    """``mq_moe_layer``: what a whole-block call needs to know about a layer."""
+    _fields_ = ([(n, c_int64) for n in ("hidden", "inter", "experts", "top_k", "group_size")]
+                + [(n, ctypes.c_int32) for n in ("dtype", "router_dtype", "renormalize", "reserved")]
+                + [("router", c_void_p), ("router_bias", c_void_p)]
+                + [(n, c_void_p * 3) for n in ("gate", "up", "down")])
+
 
 _lib = None
 launch_count = 0   # kernels launched through this binding (each wrapper adds what it launched)
@@ -98,11 +109,20 @@ def dtype_code(t: torch.Tensor) -> int:
 
 
 def ptr(t: torch.Tensor | None):
-    return None if t is None else c_void_p(t.data_ptr())
+    """The tensor's address as an int (what a ``c_void_p`` argument takes without a wrapper object)."""
+    return None if t is None else t.data_ptr()
 
 
-def stream_ptr(device) -> c_void_p:
-    return c_void_p(torch.cuda.current_stream(device).cuda_stream)
+# torch.cuda.current_stream() builds a Stream object (1.5 us); the raw handle is all a launch needs
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_ptr(device) -> int:
+    """The current stream's handle on ``device`` (a torch.device or an index)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    index = device if isinstance(device, int) else device.index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def require_cuda(*tensors: torch.Tensor) -> None:

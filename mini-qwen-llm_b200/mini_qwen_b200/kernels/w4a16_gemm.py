@@ -16,9 +16,6 @@ import torch
 from .. import _cabi
 
 
-_single_offsets: dict = {}   # (M, device) -> int32 [0, M]; a single linear is a one-expert group
-
-
 def _offsets32(expert_offsets: torch.Tensor) -> torch.Tensor:
     """The kernels read int32 offsets; ``moe_permute`` returns int64 ones, as the reference does."""
     assert expert_offsets.is_cuda, "w4a16 kernels run on CUDA tensors only"
@@ -33,13 +30,13 @@ def _check_w4(x, qweight, scales, qzeros, group_size, E, prepared_f16=False):
     assert x.dtype == (torch.float16 if prepared_f16 else torch.bfloat16), "activations must be bfloat16"
     assert qweight.dtype == torch.int32 and qzeros.dtype == torch.int32 and scales.dtype == torch.bfloat16
     K = x.shape[-1]
-    N = qweight.shape[-1]
-    assert qweight.shape[-2] * 8 == K, "qweight must be [K // 8, N]"
+    words, N = qweight.shape[-2:]
+    assert words * 8 == K, "qweight must be [K // 8, N]"
     assert K % group_size == 0, f"K={K} must be divisible by group_size={group_size}"
     assert N % 8 == 0, f"N={N} must be a multiple of 8"
     assert group_size % 32 == 0, "group_size must be a multiple of 32"
     G = K // group_size
-    assert tuple(scales.shape[-2:]) == (G, N) and tuple(qzeros.shape[-2:]) == (G, N // 8)
+    assert scales.shape[-2:] == (G, N) and qzeros.shape[-2:] == (G, N // 8)
     return K, N
 
 
@@ -122,15 +119,19 @@ def w4a16_gemm(
 ) -> torch.Tensor:
     """``x @ dequant(qweight)`` with ``W[k,n] = (q[k,n] - z[k//g,n]) * s[k//g,n]``; returns bf16 [M, N]."""
     assert x.dim() == 2 and qweight.dim() == 2
+    if not (qweight.is_contiguous() and scales.is_contiguous() and qzeros.is_contiguous()):
+        qweight, scales, qzeros = qweight.contiguous(), scales.contiguous(), qzeros.contiguous()
+    K, N = _check_w4(x, qweight, scales, qzeros, group_size, 1)
+    if not x.is_contiguous():
+        x = x.contiguous()
     M = x.shape[0]
-    key = (M, x.device)
-    offsets = _single_offsets.get(key)
-    if offsets is None:
-        if len(_single_offsets) > 256:
-            _single_offsets.clear()
-        offsets = _single_offsets[key] = torch.tensor([0, M], dtype=torch.int32, device=x.device)
-    return w4a16_grouped_gemm(x, qweight.contiguous().unsqueeze(0), scales.contiguous().unsqueeze(0),
-                              qzeros.contiguous().unsqueeze(0), offsets, group_size, zero_init=False)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    rc = _cabi.load().mq_w4a16_linear(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), M, N, K,
+                                      group_size, out.data_ptr(), _cabi.stream_ptr(x.get_device()))
+    if rc:
+        _cabi.check(rc, "mq_w4a16_linear")
+    _cabi.count_launches(1 if M else 0)
+    return out
 
 
 # ---- prepared-activation forms of the stream kernel (the block's decode path) ------------------

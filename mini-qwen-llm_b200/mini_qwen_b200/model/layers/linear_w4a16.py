@@ -29,9 +29,11 @@ class LinearW4A16(nn.Module):
         self.register_buffer("qzeros", torch.zeros(groups, out_features // 8, dtype=torch.int32))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
-        y = w4a16_gemm(x.reshape(-1, self.in_features), self.qweight, self.scales, self.qzeros, self.group_size)
-        return y.reshape(*lead, self.out_features)
+        buf = self._buffers                  # a Module's own attribute lookup costs half a microsecond a buffer
+        if x.dim() == 2 and x.shape[1] == self.in_features:
+            return w4a16_gemm(x, buf["qweight"], buf["scales"], buf["qzeros"], self.group_size)
+        y = w4a16_gemm(x.reshape(-1, self.in_features), buf["qweight"], buf["scales"], buf["qzeros"], self.group_size)
+        return y.reshape(*x.shape[:-1], self.out_features)
 
     @classmethod
     def from_float(cls, linear: nn.Linear, group_size: int = 128) -> "LinearW4A16":

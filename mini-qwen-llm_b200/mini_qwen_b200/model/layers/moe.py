@@ -12,9 +12,12 @@ device or dtype, invalidates the stacks; the next forward rebuilds them.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 import torch.nn as nn
 
+from ... import _cabi
 from ...kernels.moe_grouped_gemm import (gather_swiglu_supported, moe_grouped_gemm, moe_grouped_gemm_scatter,
                                           moe_grouped_swiglu, moe_grouped_swiglu_gather, scatter_gemm_supported)
 from ...kernels.moe_permute import gather_rows, moe_permute_plan
@@ -49,6 +52,28 @@ class _ExpertMLP(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """Single-expert path (kept for callers that address one expert; the block does not use it)."""
         return self.down_proj(nn.functional.silu(self.gate_proj(x)) * self.up_proj(x))
+
+
+class _NativeLayer:
+    """A layer's description in the library's terms, and the workspace sizes its calls have needed."""
+
+    def __init__(self, layer: _cabi.MoELayer, dtype, device: int, hidden: int):
+        self.layer, self.dtype, self.device, self.hidden = layer, dtype, device, hidden
+        self.address = ctypes.addressof(layer)
+        self.launches = ctypes.c_int32(0)
+        self.launches_address = ctypes.addressof(self.launches)
+        self._bytes: dict = {}
+
+    def workspace_bytes(self, lib, T: int) -> int:
+        n = self._bytes.get(T)
+        if n is None:
+            if len(self._bytes) > 1024:
+                self._bytes.clear()
+            n = self._bytes[T] = lib.mq_moe_forward_workspace_bytes(self.address, T)
+        return n
+
+    def __reduce__(self):     # holds addresses: a copied or loaded block makes its own
+        return type(None), ()
 
 
 class Qwen3MoEBlock(nn.Module):
@@ -108,6 +133,7 @@ class Qwen3MoEBlock(nn.Module):
         self.experts = nn.ModuleList([_ExpertMLP(config, self._epoch) for _ in range(self.num_local_experts)])
         self.router_bias = None       # optional fp32 [E] logit bias (not in the reference)
         self._status = None
+        self._native = None           # description of the layer for the whole-block call, and what it was made from
         self.kernel_events = None     # set to a list to collect (stage, start, end) CUDA events per forward
 
     # ------------------------------------------------------------------ weight stacks
@@ -116,9 +142,13 @@ class Qwen3MoEBlock(nn.Module):
         return super()._apply(fn, *args, **kwargs)
 
     def _sentinel(self):
-        first, last = self.experts[0].gate_proj, self.experts[-1].down_proj
-        a = first.qweight if isinstance(first, LinearW4A16) else first.weight
-        b = last.qweight if isinstance(last, LinearW4A16) else last.weight
+        # through the modules' own dicts: this runs on every call, and Module.__getattr__ and ModuleList indexing
+        # would take ten microseconds
+        experts = self._modules["experts"]._modules
+        first = experts["0"]._modules["gate_proj"]
+        last = experts[str(self.num_local_experts - 1)]._modules["down_proj"]
+        a = first._buffers["qweight"] if isinstance(first, LinearW4A16) else first._parameters["weight"]
+        b = last._buffers["qweight"] if isinstance(last, LinearW4A16) else last._parameters["weight"]
         return (a.data_ptr(), b.data_ptr())
 
     def finalize(self) -> None:
@@ -232,6 +262,87 @@ class Qwen3MoEBlock(nn.Module):
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         """The block on ``x`` [..., H].  With ``residual`` (same shape and dtype) the result is
         ``residual + block(x)``, the add done by the combine kernel as an add of two model-dtype tensors."""
+        if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype):
+            raise ValueError("residual must have the shape and dtype of the block's input")
+        out = self._forward_native(x, residual, None, 0.0)
+        return out if out is not None else self._forward_staged(x, residual)
+
+    def _native_layer(self):
+        """The layer's description for :func:`mq_moe_forward`, made again when anything it points to has changed; None
+        when the whole-block call does not apply (expert parallelism, stage timing, a kernel chosen by hand)."""
+        if (self.ep_size != 1 or self.kernel_events is not None or self.w4_kernel != "stream" or self.w4_rows_f16
+                or not self.fuse_small_batches or self.fuse_max_tokens != 64):
+            return None
+        st = self._ready()
+        router, bias = self._modules["gate"]._parameters["weight"], self.router_bias
+        key = (self._stacked_epoch, self._stacked_sentinel, router.data_ptr(), None if bias is None else bias.data_ptr(),
+               self.norm_topk_prob, self.num_experts_per_tok)
+        native = self._native
+        if native is not None and native[0] == key:
+            return native[1]
+        E, H = router.shape
+        made = None
+        dense = not st["w4"]
+        w = st["w13"] if dense else st["gate_proj"][0]
+        if (router.is_cuda and router.is_contiguous() and w.is_cuda and w.get_device() == router.get_device()
+                and router.dtype in _cabi._DTYPES and (not dense or w.dtype in _cabi._DTYPES)
+                and E == self.num_experts and self.num_experts_per_tok <= 32
+                and (bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.is_cuda
+                                      and bias.numel() == E))):
+            L = _cabi.MoELayer(hidden=H, experts=E, top_k=self.num_experts_per_tok, renormalize=int(self.norm_topk_prob),
+                               router_dtype=_cabi.dtype_code(router), router=router.data_ptr(),
+                               router_bias=None if bias is None else bias.data_ptr())
+            if dense:
+                L.inter, L.group_size, L.dtype = w.shape[1] // 2, 0, _cabi.dtype_code(w)
+                L.gate[0], L.down[0] = w.data_ptr(), st["w2"].data_ptr()
+            else:
+                L.inter, L.group_size, L.dtype = w.shape[2], st["group_size"], _cabi.MQ_BF16
+                for name in ("gate", "up", "down"):
+                    for i, t in enumerate(st[name + "_proj"]):
+                        getattr(L, name)[i] = t.data_ptr()
+            made = _NativeLayer(L, w.dtype if dense else torch.bfloat16, w.get_device(), H)
+        self._native = (key, made)
+        return made
+
+    def _forward_native(self, x, residual, norm_weight, norm_eps: float):
+        """The whole block in one library call, or None when it does not apply to these tensors."""
+        nat = self._native_layer()
+        if nat is None or x.dtype != nat.dtype or x.get_device() != nat.device or x.shape[-1] != nat.hidden:
+            return None
+        if not x.is_contiguous():
+            x = x.contiguous()
+        T = x.numel() // nat.hidden
+        if T == 0:
+            return None
+        if residual is not None:
+            if residual.get_device() != nat.device:
+                return None
+            if not residual.is_contiguous():
+                residual = residual.contiguous()
+        out = torch.empty_like(x)
+        route_ws = None
+        if T <= 64:
+            route_ws = self._route_ws
+            if route_ws is None or route_ws.device != x.device:
+                route_ws = self._route_ws = route_small_workspace(self.num_experts, x.device)
+        status = self._status
+        if status is None or status.device != x.device:
+            status = self._status_word(x.device)
+        lib = _cabi.load()
+        space = nat.workspace_bytes(lib, T)
+        ws = torch.empty(space, dtype=torch.uint8, device=x.device)
+        rc = lib.mq_moe_forward(nat.address, x.data_ptr(), norm_weight, norm_eps,
+                                None if residual is None else residual.data_ptr(), T,
+                                None if route_ws is None else route_ws.data_ptr(), 0 if route_ws is None else route_ws.numel(),
+                                ws.data_ptr(), space, out.data_ptr(), status.data_ptr(), nat.launches_address,
+                                _cabi.stream_ptr(nat.device))
+        if rc:
+            _cabi.check(rc, "mq_moe_forward")
+        _cabi.count_launches(nat.launches.value)
+        return out
+
+    def _forward_staged(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
+        """The same chain, stage by stage: expert parallelism, stage timing and the kernels chosen by hand."""
         shape = x.shape
         x2d = x.reshape(-1, shape[-1])
         if not x2d.is_contiguous():
@@ -239,8 +350,6 @@ class Qwen3MoEBlock(nn.Module):
         T = x2d.shape[0]
         res = None
         if residual is not None:
-            if residual.shape != x.shape or residual.dtype != x.dtype:
-                raise ValueError("residual must have the shape and dtype of the block's input")
             res = residual.reshape(-1, shape[-1]).contiguous()
         K, E = self.num_experts_per_tok, self.num_experts
         st = self._ready()
@@ -319,6 +428,13 @@ class Qwen3MoEBlock(nn.Module):
     def half_layer(self, h: torch.Tensor, norm: "RMSNorm") -> torch.Tensor:
         """Second half of the reference's MoE decoder layer (``mini_qwen/model/qwen3_moe.py:63-66``):
         ``h + self(norm(h))`` with ``norm`` the layer's post-attention RMSNorm; the add runs in the combine kernel."""
+        if type(norm) is RMSNorm and not norm._forward_hooks and not norm._forward_pre_hooks:
+            weight = norm._parameters["weight"]
+            if (weight.dtype == h.dtype and weight.shape == h.shape[-1:] and weight.is_contiguous()
+                    and weight.get_device() == h.get_device()):
+                out = self._forward_native(h, h, weight.data_ptr(), norm.eps)
+                if out is not None:
+                    return out
         return self.forward(norm(h), residual=h)
 
     def _experts(self, st, rows, off32, out=None):
