@@ -12,6 +12,10 @@
 namespace mq {
 
 bool tc5_covers(int64_t S, int64_t E, int64_t N, int64_t Kd, bool swiglu);
+bool generic_small_groups(int64_t S, int64_t E, int64_t N);
+int grouped_gemm_generic_dispatch(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E,
+                                  int64_t period, int64_t N, int64_t Kd, int dtype, bool swiglu, void* out,
+                                  cudaStream_t st, const int32_t* perm, int64_t top_k);
 bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 
@@ -19,7 +23,7 @@ namespace {
 
 // How a call runs.
 struct BlockPlan {
-  bool w4, small, prepared, tile, stream, gather_in_kernel;
+  bool w4, small, prepared, tile, stream, tc5, gather_in_kernel;
 };
 
 BlockPlan plan_of(const mq_moe_layer& L, int64_t T) {
@@ -35,7 +39,8 @@ BlockPlan plan_of(const mq_moe_layer& L, int64_t T) {
     p.prepared = p.stream && p.small && T <= E;
     p.gather_in_kernel = p.tile || p.stream;
   } else {
-    p.gather_in_kernel = L.dtype == MQ_BF16 && tc5_covers(S, E, I, H, true) && T * H < ((int64_t)1 << 32);
+    p.tc5 = L.dtype == MQ_BF16 && tc5_covers(S, E, I, H, true) && T * H < ((int64_t)1 << 32);
+    p.gather_in_kernel = p.tc5 || generic_small_groups(S, E, I);
   }
   return p;
 }
@@ -146,8 +151,11 @@ extern "C" int mq_moe_forward(const mq_moe_layer* h_layer, const void* x, const 
     ++n;
   }
   if (!p.w4) {
-    if (p.gather_in_kernel)
+    if (p.tc5)
       MQ_BLOCK_STEP(mq_grouped_swiglu_gather(x, b.perm, L.gate[0], b.offsets, T, K, E, E, I, H, L.dtype, b.h, d_status, stream));
+    else if (p.gather_in_kernel)
+      MQ_BLOCK_STEP(grouped_gemm_generic_dispatch(x, L.gate[0], b.offsets, S, E, E, I, H, L.dtype, true, b.h,
+                                                  reinterpret_cast<cudaStream_t>(stream), b.perm, K));
     else
       MQ_BLOCK_STEP(mq_grouped_swiglu(b.rows, L.gate[0], b.offsets, S, E, E, I, H, L.dtype, b.h, d_status, stream));
     MQ_BLOCK_STEP(mq_grouped_gemm(b.h, L.down[0], b.offsets, S, E, E, H, I, L.dtype, b.y, d_status, stream));

@@ -42,7 +42,7 @@ int device_sm_count() {
 
 int grouped_gemm_generic_dispatch(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E,
                                   int64_t period, int64_t N, int64_t Kd, int dtype, bool swiglu, void* out,
-                                  cudaStream_t st);
+                                  cudaStream_t st, const int32_t* perm, int64_t top_k);
 
 // tcgen05 kernel (bf16). Returns MQ_ERR_UNSUPPORTED_SHAPE when the shape is outside its cover.
 int grouped_gemm_tc5(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E, int64_t period,
@@ -83,7 +83,7 @@ static int grouped_common(const void* a, const void* w, const int32_t* offsets, 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == MQ_BF16 && tc5_covers(S, period, N, Kd, swiglu) && aligned16(a) && aligned16(w) && aligned16(out))
     return grouped_gemm_tc5(a, w, offsets, S, E, period, N, Kd, swiglu, out, d_status, st, nullptr, 1, nullptr, nullptr);
-  return grouped_gemm_generic_dispatch(a, w, offsets, S, E, period, N, Kd, dtype, swiglu, out, st);
+  return grouped_gemm_generic_dispatch(a, w, offsets, S, E, period, N, Kd, dtype, swiglu, out, st, nullptr, 1);
 }
 
 extern "C" int mq_grouped_gemm(const void* a, const void* w, const int32_t* offsets,

@@ -27,11 +27,9 @@
 //
 // Every mbarrier wait is bounded: when it runs out the kernel sets MQ_DEV_WAIT_EXPIRED in the status
 // word, all roles leave their loops, and TMEM is freed before the CTA exits.
-#include <cuda.h>
-
 #include <mutex>
 
-#include "common.cuh"
+#include "tc5.cuh"
 
 namespace mq {
 namespace {
@@ -282,7 +280,7 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(bar_mem + 8 * (2 * NST + 4));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * (2 * NST + 4) + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)tc5::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int cols_per_tile = (SWIGLU || DOUBLE) ? TM : 2 * TM;      // output columns per tile
   const int NWT = (N + cols_per_tile - 1) / cols_per_tile;
   const int KB = Kd / BK;
@@ -308,7 +306,7 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = tc5::uniform(*tmem_ptr_smem);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -352,31 +350,34 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      TileCursor cur(offsets, E, NWT);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      Tile tl;
-      int it = 0;                                  // tiles this CTA has started
-      for (int t = blockIdx.x; ok; t += gridDim.x, ++it) {
-        if (!cur.locate(t, tl)) break;
-        const bool two = !DOUBLE && (SWIGLU || (tl.wt * cols_per_tile + TM < N));
-        const uint32_t idesc = umma_idesc(tl.n_mma);
-        const int buf = DOUBLE ? (it & 1) : 0;     // accumulator of this tile
-        const uint32_t acc_phase = (uint32_t)((DOUBLE ? (it >> 1) : it) & 1);
-        const uint32_t acc = tmem_base + buf * TN_MAX;
-        ok = mbar_wait(tempty_bar(buf), acc_phase ^ 1u, abort_flag, d_status);   // epilogue has drained it
+    // The whole warp walks the loop and one elected lane issues, so that addresses and descriptors stay in uniform
+    // registers; a loop that a single lane runs pays for every MMA what moving them there costs.
+    const bool leader = tc5::elect_one();
+    TileCursor cur(offsets, E, NWT);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    Tile tl;
+    int it = 0;                                  // tiles this CTA has started
+    for (int t = blockIdx.x; ok; t += gridDim.x, ++it) {
+      if (!cur.locate(t, tl)) break;
+      const bool two = !DOUBLE && (SWIGLU || (tl.wt * cols_per_tile + TM < N));
+      const uint32_t idesc = tc5::uniform(umma_idesc(tl.n_mma));
+      const int buf = DOUBLE ? (it & 1) : 0;     // accumulator of this tile
+      const uint32_t acc_phase = (uint32_t)((DOUBLE ? (it >> 1) : it) & 1);
+      const uint32_t acc = tmem_base + buf * TN_MAX;
+      ok = tc5::mbar_wait_warp(tempty_bar(buf), acc_phase ^ 1u, abort_flag, d_status);   // epilogue has drained it
+      if (!ok) break;
+      tc_fence_after();
+      for (int kb = 0; kb < KB; ++kb) {
+        ok = tc5::mbar_wait_warp(full_bar(stage), phase, abort_flag, d_status);
         if (!ok) break;
         tc_fence_after();
-        for (int kb = 0; kb < KB; ++kb) {
-          ok = mbar_wait(full_bar(stage), phase, abort_flag, d_status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t sa0 = tiles_base + stage * SBYTES;
-          const uint64_t a0 = umma_desc(sa0);
-          const uint64_t a1 = umma_desc(sa0 + A_BYTES);
-          const uint64_t bd = umma_desc(sa0 + B_OFF);
+        const uint32_t sa0 = tiles_base + stage * SBYTES;
+        const uint64_t a0 = umma_desc(sa0);
+        const uint64_t a1 = umma_desc(sa0 + A_BYTES);
+        const uint64_t bd = umma_desc(sa0 + B_OFF);
+        if (leader) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             // 16 k = 32 bytes along the swizzled row: +2 in the (address >> 4) field
@@ -385,11 +386,13 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             if (two) umma_f16(acc + TN_MAX, a1 + 2u * k, bd + 2u * k, idesc, accum);
           }
           umma_commit(empty_bar(stage));          // frees the ring slot once these MMAs have read it
-          if (++stage == NST) { stage = 0; phase ^= 1u; }
         }
-        if (!ok) break;
-        umma_commit(tfull_bar(buf));              // accumulators complete
+        __syncwarp();
+        if (++stage == NST) { stage = 0; phase ^= 1u; }
       }
+      if (!ok) break;
+      if (leader) umma_commit(tfull_bar(buf));    // accumulators complete
+      __syncwarp();
     }
   } else if (GATHER && warp >= 2 + EPI_WARPS) {
     // ------------------------------------------------------------------ gather producers (warps 10..13)

@@ -466,9 +466,9 @@ __device__ void route_prepare_row(const __nv_bfloat16* __restrict__ x_row, int H
 constexpr int RTK_THREADS = 256;
 constexpr int RTK_HEADER_INTS = 128;                  // workspace header: counter of the narrow kernel, all-tokens
                                                       // counter, one counter per token (64)
-template <int EPL>
+template <int EPL, bool F32>
 __global__ void __launch_bounds__(RTK_THREADS)
-route_tokens_kernel(const uint16_t* __restrict__ x, int x_bf16, const uint16_t* __restrict__ w, int w_bf16,
+route_tokens_kernel(const void* __restrict__ xv_, int xdt, const void* __restrict__ wv_, int wdt,
                     const float* __restrict__ bias, int T, int H, int E, int K, int renorm,
                     float* __restrict__ logits, int* __restrict__ header,
                     int32_t* __restrict__ ids32, int64_t* __restrict__ ids64, float* __restrict__ weights,
@@ -485,38 +485,55 @@ route_tokens_kernel(const uint16_t* __restrict__ x, int x_bf16, const uint16_t* 
   pdl_wait();
   pdl_release();
 
-  // ---- logits: warp `warp` takes experts e0 .. e0+3; a lane's pieces of the row: k = 8 (lane + 32 i)
+  // ---- logits: warp `warp` takes experts e0, e0 + 8, e0 + 16, e0 + 24; a lane's pieces of the row: k = 8 (lane + 32 i)
   {
     constexpr int MAXP = 8;                            // pieces per lane kept in registers (H <= 2048); more: re-read
     const int pieces = H / 8;
-    const uint16_t* xr = x + (size_t)t * H;
-    const int e0 = eg * 32 + warp * 4;
+    const int e0 = eg * 32 + warp;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int p0 = 0; p0 < pieces; p0 += 32 * MAXP) {
-      uint4 xv[MAXP];
+    if (F32) {
+      for (int pc = lane; pc < pieces; pc += 32) {
+        float a[8], b[4][8];
+        load8(xv_, xdt, (size_t)t * H + 8 * pc, a);
 #pragma unroll
-      for (int i = 0; i < MAXP; ++i) {
-        const int pc = p0 + lane + 32 * i;
-        xv[i] = pc < pieces ? __ldg(reinterpret_cast<const uint4*>(xr) + pc) : make_uint4(0, 0, 0, 0);
-      }
+        for (int j = 0; j < 4; ++j)
+          if (e0 + 8 * j < E) load8(wv_, wdt, (size_t)(e0 + 8 * j) * H + 8 * pc, b[j]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int e = e0 + j;
-        if (e < E) {
-          const uint4* wr = reinterpret_cast<const uint4*>(w + (size_t)e * H);
-          uint4 wv[MAXP];
+        for (int j = 0; j < 4; ++j)
+          if (e0 + 8 * j < E) {
 #pragma unroll
-          for (int i = 0; i < MAXP; ++i) {
-            const int pc = p0 + lane + 32 * i;
-            wv[i] = pc < pieces ? __ldg(wr + pc) : make_uint4(0, 0, 0, 0);
+            for (int q = 0; q < 8; ++q) acc[j] = fmaf(a[q], b[j][q], acc[j]);
           }
+      }
+    } else {
+      const uint16_t* xr = reinterpret_cast<const uint16_t*>(xv_) + (size_t)t * H;
+      const uint16_t* w = reinterpret_cast<const uint16_t*>(wv_);
+      for (int p0 = 0; p0 < pieces; p0 += 32 * MAXP) {
+        uint4 xv[MAXP];
 #pragma unroll
-          for (int i = 0; i < MAXP; ++i) {
-            float a[8], b[8];
-            unpack8_16bit(xv[i], x_bf16 != 0, a);
-            unpack8_16bit(wv[i], w_bf16 != 0, b);
+        for (int i = 0; i < MAXP; ++i) {
+          const int pc = p0 + lane + 32 * i;
+          xv[i] = pc < pieces ? __ldg(reinterpret_cast<const uint4*>(xr) + pc) : make_uint4(0, 0, 0, 0);
+        }
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc[j] = fmaf(a[q], b[q], acc[j]);
+        for (int j = 0; j < 4; ++j) {
+          const int e = e0 + 8 * j;
+          if (e < E) {
+            const uint4* wr = reinterpret_cast<const uint4*>(w + (size_t)e * H);
+            uint4 wv[MAXP];
+#pragma unroll
+            for (int i = 0; i < MAXP; ++i) {
+              const int pc = p0 + lane + 32 * i;
+              wv[i] = pc < pieces ? __ldg(wr + pc) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < MAXP; ++i) {
+              float a[8], b[8];
+              unpack8_16bit(xv[i], xdt == MQ_BF16, a);
+              unpack8_16bit(wv[i], wdt == MQ_BF16, b);
+#pragma unroll
+              for (int q = 0; q < 8; ++q) acc[j] = fmaf(a[q], b[q], acc[j]);
+            }
           }
         }
       }
@@ -526,20 +543,23 @@ route_tokens_kernel(const uint16_t* __restrict__ x, int x_bf16, const uint16_t* 
       float v = acc[j];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0 && e0 + j < E) logits[(size_t)t * E + e0 + j] = v;
+      if (lane == 0 && e0 + 8 * j < E) logits[(size_t)t * E + e0 + 8 * j] = v;
     }
   }
   if (xp != nullptr && eg == 0)
-    route_prepare_row(reinterpret_cast<const __nv_bfloat16*>(x) + (size_t)t * H, H, prep_mode, xp + (size_t)t * H,
+    route_prepare_row(reinterpret_cast<const __nv_bfloat16*>(xv_) + (size_t)t * H, H, prep_mode, xp + (size_t)t * H,
                       xs + (size_t)t * W4_XS_STRIDE, s_red);
 
-  // ---- last on this token?
+  // ---- last on this token?  (at most 32 experts: this CTA formed all of the token's logits)
+  if (groups > 1) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&tok_ctr[t], 1) == groups - 1;
+    __syncthreads();
+    if (!s_last) return;
+  }
   __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(&tok_ctr[t], 1) == groups - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
   unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(rtk_smem);   // [E]
   float* s_logits = reinterpret_cast<float*>(s_mask + E);                        // [E]
   int* s_ids = reinterpret_cast<int*>(s_logits + E);                             // [T * K]
@@ -878,20 +898,27 @@ extern "C" int mq_route_small(const void* x, int x_dtype, const void* w, int w_d
   int* counter = reinterpret_cast<int*>(workspace);
   float* logits = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + RTK_HEADER_INTS * sizeof(int));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (T > 16 && vec_ok && x_dtype != MQ_F32 && w_dtype != MQ_F32) {
-    // more tokens than one CTA has warps: the token-major kernel (selection on as many SMs as there are tokens)
+  if (vec_ok && (T > 16 || E <= 32)) {
+    // The token-major kernel (selection on as many SMs as there are tokens) where one CTA has fewer warps than there
+    // are tokens, or where few experts leave the expert-major kernel with a handful of CTAs (fp32 layer, 8 experts, 64
+    // tokens: 17.3 us there, one CTA per expert).
     const size_t smem_t = (size_t)E * 8 + (size_t)E * 4 + (size_t)T * K * 4 + (size_t)E * 4;
     const dim3 grid((unsigned)((E + 31) / 32), (unsigned)T);
 #define MQ_RTK_LAUNCH(EPL)                                                                                       \
-    launch_after_predecessor(route_tokens_kernel<EPL>, grid, dim3(RTK_THREADS), smem_t, st,                       \
-        reinterpret_cast<const uint16_t*>(x), (int)(x_dtype == MQ_BF16), reinterpret_cast<const uint16_t*>(w),    \
-        (int)(w_dtype == MQ_BF16), bias, (int)T, (int)H, (int)E, (int)K, renormalize, logits, counter, ids32,     \
+  do {                                                                                                           \
+    if (x_dtype != MQ_F32 && w_dtype != MQ_F32) MQ_RTK_LAUNCH2(EPL, false);                                      \
+    else MQ_RTK_LAUNCH2(EPL, true);                                                                              \
+  } while (0)
+#define MQ_RTK_LAUNCH2(EPL, F32)                                                                                 \
+    launch_after_predecessor(route_tokens_kernel<EPL, F32>, grid, dim3(RTK_THREADS), smem_t, st, x, x_dtype, w,   \
+        w_dtype, bias, (int)T, (int)H, (int)E, (int)K, renormalize, logits, counter, ids32,                      \
         ids64, weights, perm, inv, offsets32, offsets64, reinterpret_cast<__nv_bfloat16*>(xp), xs,                \
         xp_format == 2 ? 2 : 1)
     if (E <= 32) MQ_RTK_LAUNCH(1);
     else if (E <= 64) MQ_RTK_LAUNCH(2);
     else if (E <= 128) MQ_RTK_LAUNCH(4);
     else MQ_RTK_LAUNCH(8);
+#undef MQ_RTK_LAUNCH2
 #undef MQ_RTK_LAUNCH
     return check_launch();
   }
