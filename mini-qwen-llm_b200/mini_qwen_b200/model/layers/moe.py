@@ -54,6 +54,10 @@ class _ExpertMLP(nn.Module):
         return self.down_proj(nn.functional.silu(self.gate_proj(x)) * self.up_proj(x))
 
 
+def _layout(t: torch.Tensor):
+    return t.data_ptr(), t.dtype, t.shape, t.stride(), t.get_device()
+
+
 class _NativeLayer:
     """A layer's description in the library's terms, and the workspace sizes its calls have needed."""
 
@@ -275,7 +279,8 @@ class Qwen3MoEBlock(nn.Module):
             return None
         st = self._ready()
         router, bias = self._modules["gate"]._parameters["weight"], self.router_bias
-        key = (self._stacked_epoch, self._stacked_sentinel, router.data_ptr(), None if bias is None else bias.data_ptr(),
+        # the layouts beside the addresses: another view of the same storage, or a tensor at a freed one's place
+        key = (self._stacked_epoch, self._stacked_sentinel, _layout(router), None if bias is None else _layout(bias),
                self.norm_topk_prob, self.num_experts_per_tok)
         native = self._native
         if native is not None and native[0] == key:

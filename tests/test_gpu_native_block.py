@@ -54,6 +54,10 @@ def test_description_follows_the_layer():
     blk(x)
     blk.gate.weight = torch.nn.Parameter(-blk.gate.weight.data, requires_grad=False)
     assert torch.equal(blk(x), blk._forward_staged(x))
+    rows = blk.gate.weight.data
+    blk.gate.weight.data = rows.as_strided((8, 128), (1, 8))        # another layout at the same address
+    assert torch.equal(blk(x), blk._forward_staged(x))
+    blk.gate.weight.data = rows
     blk.router_bias = torch.linspace(1, -1, 8, device=DEV)
     assert torch.equal(blk(x), blk._forward_staged(x))
     blk.experts[0].gate_proj.weight.data = blk.experts[0].gate_proj.weight.data * 2
