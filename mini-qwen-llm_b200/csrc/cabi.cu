@@ -50,6 +50,12 @@ int grouped_gemm_tc5(const void* a, const void* w, const int32_t* offsets, int64
                      const int32_t* perm, int64_t top_k, const int32_t* row_dst, const uint64_t* dst_bases);
 bool tc5_covers(int64_t S, int64_t E, int64_t N, int64_t Kd, bool swiglu);
 
+// The same on CTA pairs: the faster one wherever it says that it covers the shape (measured at its definition).
+bool grouped_gemm_pair_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, bool swiglu);
+int grouped_gemm_pair(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E, int64_t period,
+                      int64_t N, int64_t Kd, bool swiglu, void* out, int32_t* d_status, cudaStream_t st,
+                      const int32_t* perm, int64_t top_k);
+
 }  // namespace mq
 
 extern "C" int mq_version(void) { return 1; }
@@ -81,7 +87,10 @@ static int grouped_common(const void* a, const void* w, const int32_t* offsets, 
   if (S == 0) return MQ_OK;
   if (!a || !w || !offsets || !out) return MQ_ERR_INVALID_ARGUMENT;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == MQ_BF16 && tc5_covers(S, period, N, Kd, swiglu) && aligned16(a) && aligned16(w) && aligned16(out))
+  const bool aligned = aligned16(a) && aligned16(w) && aligned16(out);
+  if (dtype == MQ_BF16 && aligned && grouped_gemm_pair_covers(S, E, period, N, Kd, swiglu))
+    return grouped_gemm_pair(a, w, offsets, S, E, period, N, Kd, swiglu, out, d_status, st, nullptr, 1);
+  if (dtype == MQ_BF16 && aligned && tc5_covers(S, period, N, Kd, swiglu))
     return grouped_gemm_tc5(a, w, offsets, S, E, period, N, Kd, swiglu, out, d_status, st, nullptr, 1, nullptr, nullptr);
   return grouped_gemm_generic_dispatch(a, w, offsets, S, E, period, N, Kd, dtype, swiglu, out, st, nullptr, 1);
 }
@@ -112,6 +121,9 @@ extern "C" int mq_grouped_swiglu_gather(const void* x, const int32_t* perm, cons
   if (S == 0) return MQ_OK;
   if (!x || !perm || !w_gate_up || !offsets || !h) return MQ_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(w_gate_up) || !aligned16(h)) return MQ_ERR_INVALID_ARGUMENT;
+  if (grouped_gemm_pair_covers(S, E, weight_period, I, H, true))
+    return grouped_gemm_pair(x, w_gate_up, offsets, S, E, weight_period, I, H, true, h, d_status,
+                             reinterpret_cast<cudaStream_t>(stream), perm, top_k);
   return grouped_gemm_tc5(x, w_gate_up, offsets, S, E, weight_period, I, H, true, h, d_status,
                           reinterpret_cast<cudaStream_t>(stream), perm, top_k, nullptr, nullptr);
 }
