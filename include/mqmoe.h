@@ -135,6 +135,12 @@ int mq_permute_plan(const void* ids, int ids_are_64, int64_t T, int64_t K, int64
                     int32_t* perm, int32_t* inv, int64_t* offsets64, int32_t* offsets32,
                     void* workspace, size_t workspace_bytes, void* stream);
 
+/* What a grouped GEMM wants beforehand (moe_grouped_gemm.py:133-137 allocates a zeroed result): zeros in the rows of
+ * out [S, N] that no group of the E + 1 offsets covers (out may be null), the offsets as 32-bit numbers (offsets32 [E + 1],
+ * may be null), the status word cleared (may be null). */
+int mq_grouped_prepare(const void* offsets, int offsets_are_64, int64_t S, int64_t E, int64_t N, int dtype, void* out,
+                       int32_t* offsets32, int32_t* d_status, void* stream);
+
 /* Row gather of moe_permute (moe_permute.py:30-31): out[p,:] = x[perm[p] / K, :].
  * H * sizeof(dtype) must be a multiple of 16 and the pointers 16-byte aligned. */
 int mq_gather_rows(const void* x, int dtype, const int32_t* perm, int64_t S, int64_t K, int64_t H,

@@ -139,6 +139,44 @@ gather_rows_bytes(const uint8_t* __restrict__ x, const int32_t* __restrict__ per
 }
 
 // ---------------------------------------------------------------------------------------------
+// What a single grouped GEMM wants beforehand, in one launch: the offsets in 32 bits, a cleared status word, and zeros in
+// the rows that no group covers.  Offsets that run from 0 to S cover every row, so usually nothing is written; filling the
+// whole result first, converting the offsets and clearing the word were three launches and a pass over memory
+// (5.2 + 1.8 + 1.2 us for 6216 rows of 768).
+template <bool OFF64>
+__global__ void __launch_bounds__(256)
+grouped_prepare(const void* __restrict__ offsets, int E, int64_t S, int64_t row_bytes, int vec, uint8_t* __restrict__ out,
+                int32_t* __restrict__ off32, int32_t* __restrict__ status) {
+  auto off = [&](int e) {
+    return OFF64 ? reinterpret_cast<const int64_t*>(offsets)[e] : (int64_t)reinterpret_cast<const int32_t*>(offsets)[e];
+  };
+  if (blockIdx.x == 0) {
+    if (off32 != nullptr)
+      for (int e = threadIdx.x; e <= E; e += 256) off32[e] = (int32_t)off(e);
+    if (status != nullptr && threadIdx.x == 0) *status = 0;
+  }
+  if (out == nullptr) return;
+  // a row between the first and the last offset lies in some group
+  const int64_t lo = off(0), hi = off(E);
+  if (lo <= 0 && hi >= S) return;
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < S; r += (int64_t)gridDim.x * 8) {
+    bool covered = r >= lo && r < hi;
+    if (!covered) {
+      for (int e = lane; e < E; e += 32) covered = covered || (off(e) <= r && r < off(e + 1));
+      covered = __any_sync(0xffffffffu, covered);
+    }
+    if (covered) continue;
+    uint8_t* o = out + r * row_bytes;
+    if (vec) {
+      for (int64_t i = lane; i < row_bytes / 16; i += 32) reinterpret_cast<uint4*>(o)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+      for (int64_t i = lane; i < row_bytes; i += 32) o[i] = 0;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // out[t,h] = cast( sum_k w[t,k] * float(rows[inv[t*K+k], h]) ): the product is rounded to fp32
 // before the add (no FMA contraction), k ascending, as a tensor multiply followed by sum(dim=1).
 // With `residual` the decoder layer's add follows (mini_qwen/model/qwen3_moe.py:66): the block output is
@@ -246,6 +284,22 @@ extern "C" int mq_permute_plan(const void* ids, int ids_are_64, int64_t T, int64
     permute_place<true><<<nseg, P_THREADS, 0, st>>>(ids, S, (int)E, nseg, seg_hist, totals, offsets64, offsets32, perm, inv);
   else
     permute_place<false><<<nseg, P_THREADS, 0, st>>>(ids, S, (int)E, nseg, seg_hist, totals, offsets64, offsets32, perm, inv);
+  return check_launch();
+}
+
+extern "C" int mq_grouped_prepare(const void* offsets, int offsets_are_64, int64_t S, int64_t E, int64_t N, int dtype,
+                                  void* out, int32_t* offsets32, int32_t* d_status, void* stream) {
+  using namespace mq;
+  if (S < 0 || E <= 0 || N <= 0 || E >= ((int64_t)1 << 31) || !valid_dtype(dtype) || !offsets) return MQ_ERR_INVALID_ARGUMENT;
+  if (S == 0) out = nullptr;
+  const int64_t row_bytes = N * (int64_t)dtype_size(dtype);
+  const int vec = row_bytes % 16 == 0 && aligned16(out);
+  const int64_t need = out != nullptr ? (S + 7) / 8 : 1;
+  const unsigned blocks = (unsigned)(need < 592 ? need : 592);            // four to an SM
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  uint8_t* o = reinterpret_cast<uint8_t*>(out);
+  if (offsets_are_64) grouped_prepare<true><<<blocks, 256, 0, st>>>(offsets, (int)E, S, row_bytes, vec, o, offsets32, d_status);
+  else grouped_prepare<false><<<blocks, 256, 0, st>>>(offsets, (int)E, S, row_bytes, vec, o, offsets32, d_status);
   return check_launch();
 }
 

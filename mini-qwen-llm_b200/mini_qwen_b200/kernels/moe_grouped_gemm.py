@@ -39,16 +39,32 @@ def moe_grouped_gemm(
     a = permuted_hidden.contiguous()
     w = expert_weights.contiguous()
     S = a.shape[0]
+    lib = _cabi.load()
+    zero = out is None and zero_init
     if out is None:
-        out = (torch.zeros if zero_init else torch.empty)(S, D, dtype=a.dtype, device=a.device)
+        out = torch.empty(S, D, dtype=a.dtype, device=a.device)
     assert out.is_contiguous() and tuple(out.shape) == (S, D) and out.dtype == a.dtype
-    if status is None:
-        status = _status_word(a.device)
-    rc = _cabi.load().mq_grouped_gemm(_cabi.ptr(a), _cabi.ptr(w), _cabi.ptr(_offsets32(expert_offsets)), S, groups, E, D, H,
-                                      _cabi.dtype_code(a), _cabi.ptr(out), _cabi.ptr(status),
-                                      _cabi.stream_ptr(a.device))
+    offsets = expert_offsets if expert_offsets.dtype in (torch.int32, torch.int64) else expert_offsets.to(torch.int32)
+    offsets = offsets.contiguous()
+    wide = offsets.dtype == torch.int64
+    launches = 1
+    if S and D and groups and (zero or wide or status is None):
+        # one launch: uncovered rows zeroed, offsets narrowed, status word cleared
+        words = torch.empty(groups + 2, dtype=torch.int32, device=a.device)
+        off32 = words[1:] if wide else offsets
+        rc = lib.mq_grouped_prepare(_cabi.ptr(offsets), int(wide), S, groups, D, _cabi.dtype_code(a),
+                                    _cabi.ptr(out) if zero else None, _cabi.ptr(off32) if wide else None,
+                                    _cabi.ptr(words) if status is None else None, _cabi.stream_ptr(a.device))
+        _cabi.check(rc, "mq_grouped_prepare")
+        offsets, launches = off32, 2
+        if status is None:
+            status = words
+    elif wide or status is None:
+        offsets, status = _offsets32(offsets), _status_word(a.device) if status is None else status
+    rc = lib.mq_grouped_gemm(_cabi.ptr(a), _cabi.ptr(w), _cabi.ptr(offsets), S, groups, E, D, H,
+                             _cabi.dtype_code(a), _cabi.ptr(out), _cabi.ptr(status), _cabi.stream_ptr(a.device))
     _cabi.check(rc, "mq_grouped_gemm")
-    _cabi.count_launches(1 if S else 0)
+    _cabi.count_launches(launches if S else 0)
     return out
 
 
