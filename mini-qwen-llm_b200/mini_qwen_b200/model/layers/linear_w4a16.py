@@ -29,10 +29,14 @@ class LinearW4A16(nn.Module):
         self.register_buffer("qzeros", torch.zeros(groups, out_features // 8, dtype=torch.int32))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        buf = self._buffers                  # a Module's own attribute lookup costs half a microsecond a buffer
+        try:
+            buf = self._buffers              # a Module's own attribute lookup costs half a microsecond a buffer
+            qweight, scales, qzeros = buf["qweight"], buf["scales"], buf["qzeros"]
+        except KeyError:                     # not kept there: parametrizations, buffers turned into parameters
+            qweight, scales, qzeros = self.qweight, self.scales, self.qzeros
         if x.dim() == 2 and x.shape[1] == self.in_features:
-            return w4a16_gemm(x, buf["qweight"], buf["scales"], buf["qzeros"], self.group_size)
-        y = w4a16_gemm(x.reshape(-1, self.in_features), buf["qweight"], buf["scales"], buf["qzeros"], self.group_size)
+            return w4a16_gemm(x, qweight, scales, qzeros, self.group_size)
+        y = w4a16_gemm(x.reshape(-1, self.in_features), qweight, scales, qzeros, self.group_size)
         return y.reshape(*x.shape[:-1], self.out_features)
 
     @classmethod

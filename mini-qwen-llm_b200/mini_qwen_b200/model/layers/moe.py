@@ -148,11 +148,16 @@ class Qwen3MoEBlock(nn.Module):
     def _sentinel(self):
         # through the modules' own dicts: this runs on every call, and Module.__getattr__ and ModuleList indexing
         # would take ten microseconds
-        experts = self._modules["experts"]._modules
-        first = experts["0"]._modules["gate_proj"]
-        last = experts[str(self.num_local_experts - 1)]._modules["down_proj"]
-        a = first._buffers["qweight"] if isinstance(first, LinearW4A16) else first._parameters["weight"]
-        b = last._buffers["qweight"] if isinstance(last, LinearW4A16) else last._parameters["weight"]
+        try:
+            experts = self._modules["experts"]._modules
+            first = experts["0"]._modules["gate_proj"]
+            last = experts[str(self.num_local_experts - 1)]._modules["down_proj"]
+            a = first._buffers["qweight"] if isinstance(first, LinearW4A16) else first._parameters["weight"]
+            b = last._buffers["qweight"] if isinstance(last, LinearW4A16) else last._parameters["weight"]
+        except KeyError:        # not kept there: parametrizations, weight norm, wrapped modules, replicas
+            first, last = self.experts[0].gate_proj, self.experts[-1].down_proj
+            a = first.qweight if isinstance(first, LinearW4A16) else first.weight
+            b = last.qweight if isinstance(last, LinearW4A16) else last.weight
         return (a.data_ptr(), b.data_ptr())
 
     def finalize(self) -> None:
@@ -273,12 +278,16 @@ class Qwen3MoEBlock(nn.Module):
 
     def _native_layer(self):
         """The layer's description for :func:`mq_moe_forward`, made again when anything it points to has changed; None
-        when the whole-block call does not apply (expert parallelism, stage timing, a kernel chosen by hand)."""
+        when the whole-block call does not apply (expert parallelism, stage timing, a kernel chosen by hand, a router
+        weight that its module computes: the description holds addresses, the module has to hold the tensor)."""
         if (self.ep_size != 1 or self.kernel_events is not None or self.w4_kernel != "stream" or self.w4_rows_f16
                 or not self.fuse_small_batches or self.fuse_max_tokens != 64):
             return None
+        gate = self._modules.get("gate")
+        router, bias = None if gate is None else gate._parameters.get("weight"), self.router_bias
+        if router is None:
+            return None
         st = self._ready()
-        router, bias = self._modules["gate"]._parameters["weight"], self.router_bias
         # the layouts beside the addresses: another view of the same storage, or a tensor at a freed one's place
         key = (self._stacked_epoch, self._stacked_sentinel, _layout(router), None if bias is None else _layout(bias),
                self.norm_topk_prob, self.num_experts_per_tok)

@@ -201,3 +201,44 @@ def test_decode_replication_entry_points_reject_bad_arguments_without_a_gpu():
     assert lib.mq_rms_norm(None, 1, None, 1e-6, 4, 2048, None, None) == 1                            # null pointers
     assert lib.mq_rms_norm(None, 1, None, 1e-6, 0, 2048, None, None) == 0                            # nothing to do
     assert lib.mq_unpermute_combine_residual(None, 1, None, None, None, 4, 33, 64, None, None) == 2  # K > 32
+
+
+def _small_block(quantised=False):
+    blk = Qwen3MoEBlock(Qwen3MoEConfig(hidden_size=64, intermediate_size=32, num_experts=2, num_experts_per_tok=1))
+    if quantised:
+        blk.quantize_to_w4a16(group_size=32)
+    return blk
+
+
+@pytest.mark.parametrize("quantised", [False, True])
+@pytest.mark.parametrize("where", ["router", "expert", "weight_norm", "replica"])
+def test_weights_that_their_modules_do_not_keep_under_their_own_name(quantised, where):
+    """A parametrised router or expert projection, old-style weight norm, and the plain-attribute weights of a
+    DataParallel replica: found through the attribute, and a router that is computed on access (whose address a
+    description must not keep) goes stage by stage."""
+    blk = _small_block(quantised)
+    if where == "router":
+        nn.utils.parametrize.register_parametrization(blk.gate, "weight", nn.Identity())
+    elif where == "expert":
+        nn.utils.parametrize.register_parametrization(blk.experts[0].gate_proj, "qweight" if quantised else "weight",
+                                                      nn.Identity())
+    elif where == "weight_norm":
+        blk.gate = nn.utils.weight_norm(blk.gate)
+    else:
+        for m in blk.modules():
+            for name, p in list(m._parameters.items()):
+                if p is not None:
+                    del m._parameters[name]
+                    setattr(m, name, p.data)
+    assert len(blk._sentinel()) == 2 and blk._ready() is blk._stacks
+    assert blk._native_layer() is None                       # CPU tensors, or a router its module does not keep
+    dt = torch.bfloat16 if quantised else torch.float32
+    with pytest.raises((ValueError, AssertionError), match="CUDA"):
+        blk(torch.zeros(3, 64, dtype=dt))                    # the error of CPU tensors, not a missing name
+
+
+def test_linear_w4a16_with_a_parametrised_buffer():
+    lin = LinearW4A16(64, 32, 32)
+    nn.utils.parametrize.register_parametrization(lin, "scales", nn.Identity())
+    with pytest.raises(AssertionError, match="CUDA"):
+        lin(torch.zeros(3, 64, dtype=torch.bfloat16))
