@@ -54,6 +54,13 @@ class _ExpertMLP(nn.Module):
         return self.down_proj(nn.functional.silu(self.gate_proj(x)) * self.up_proj(x))
 
 
+def _any_module_hook() -> bool:
+    """Whether a hook is registered for all modules (``torch.nn.modules.module.register_module_*_hook``)."""
+    m = nn.modules.module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks
+                or m._global_backward_pre_hooks)
+
+
 def _layout(t: torch.Tensor):
     return t.data_ptr(), t.dtype, t.shape, t.stride(), t.get_device()
 
@@ -442,11 +449,13 @@ class Qwen3MoEBlock(nn.Module):
     def half_layer(self, h: torch.Tensor, norm: "RMSNorm") -> torch.Tensor:
         """Second half of the reference's MoE decoder layer (``mini_qwen/model/qwen3_moe.py:63-66``):
         ``h + self(norm(h))`` with ``norm`` the layer's post-attention RMSNorm; the add runs in the combine kernel."""
-        if type(norm) is RMSNorm and not norm._forward_hooks and not norm._forward_pre_hooks:
-            weight = norm._parameters["weight"]
+        weight = norm._parameters.get("weight") if type(norm) is RMSNorm else None
+        # only where calling the module would do nothing but its own forward
+        if not (weight is None or norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks
+                or norm._backward_pre_hooks or "forward" in norm.__dict__ or _any_module_hook()):
             if (weight.dtype == h.dtype and weight.shape == h.shape[-1:] and weight.is_contiguous()
                     and weight.get_device() == h.get_device()):
-                out = self._forward_native(h, h, weight.data_ptr(), norm.eps)
+                out = self._forward_native(h, h, weight.data_ptr(), float(norm.eps))
                 if out is not None:
                     return out
         return self.forward(norm(h), residual=h)

@@ -12,7 +12,7 @@ import torch.nn as nn
 import cases
 from mini_qwen_b200 import Qwen3MoEConfig, _cabi
 from mini_qwen_b200.kernels import moe_grouped_gemm, moe_permute, moe_router, moe_unpermute, w4a16_gemm
-from mini_qwen_b200.model.layers import LinearW4A16, Qwen3MoEBlock
+from mini_qwen_b200.model.layers import LinearW4A16, Qwen3MoEBlock, RMSNorm
 from mini_qwen_b200.quantization import _per_group_minmax_quantize, pack_int4, quantize_awq, unpack_int4
 from oracle import moe_oracle as O
 
@@ -242,3 +242,34 @@ def test_linear_w4a16_with_a_parametrised_buffer():
     nn.utils.parametrize.register_parametrization(lin, "scales", nn.Identity())
     with pytest.raises(AssertionError, match="CUDA"):
         lin(torch.zeros(3, 64, dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("what", ["plain", "hook", "global hook", "replica", "own forward"])
+def test_half_layer_calls_a_norm_that_does_more_than_normalise(what):
+    blk, norm = _small_block(), RMSNorm(64)
+    native = []
+    blk._forward_native = lambda h, residual, weight, eps: native.append(weight) or h
+    blk.forward = lambda h, residual: "called"
+    handle = None
+    if what == "hook":
+        norm.register_forward_hook(lambda m, i, o: None)
+    elif what == "global hook":
+        handle = nn.modules.module.register_module_forward_pre_hook(lambda m, i: None)
+    elif what == "replica":
+        w = norm._parameters.pop("weight").data
+        norm.weight = w
+    elif what == "own forward":
+        norm.forward = lambda h: h
+    h = torch.zeros(3, 64)
+    try:
+        if what == "plain":
+            assert blk.half_layer(h, norm) is h and native == [norm.weight.data_ptr()]
+        elif what == "own forward":
+            assert blk.half_layer(h, norm) == "called" and not native
+        else:
+            with pytest.raises(ValueError, match="CUDA"):    # the norm itself ran, on CPU tensors
+                blk.half_layer(h, norm)
+            assert not native
+    finally:
+        if handle is not None:
+            handle.remove()
