@@ -203,6 +203,7 @@ class Qwen3MoEBlock(nn.Module):
                     ex.down_proj.weight.data = w2[e]
                 stacks["w13"], stacks["w2"] = w13, w2
         self._stacks = stacks
+        self._native = None           # it holds the old stacks' addresses
         self._stacked_epoch = self._epoch[0]
         self._stacked_sentinel = self._sentinel()
 

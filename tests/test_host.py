@@ -273,3 +273,14 @@ def test_half_layer_calls_a_norm_that_does_more_than_normalise(what):
     finally:
         if handle is not None:
             handle.remove()
+
+
+@pytest.mark.parametrize("quantised", [False, True])
+def test_finalize_drops_the_description_of_the_old_stacks(quantised):
+    """A description holds the addresses of up to nine stacks; the two that are compared on each call may come out
+    of the allocator where they were while the others have moved."""
+    blk = _small_block(quantised)
+    blk._native_layer()
+    assert blk._native is not None
+    blk.finalize()
+    assert blk._native is None
