@@ -51,7 +51,8 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
       : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
   return ok != 0;
 }
-// Bounded wait by one thread: false (and the status bit set) when it ran out or another role of the CTA gave up.
+// Bounded wait by one thread: false, with the status bit set, when it ran out.  Nothing ends a wait early: when one
+// role gives up, the others find out by their own waits, and only the first sets the bit.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* d_status) {
   if (mbar_wait_limited(bar, parity, SPIN_LIMIT)) return true;
   if (!*abort_flag && d_status != nullptr) atomicOr(d_status, (int)MQ_DEV_WAIT_EXPIRED);

@@ -262,19 +262,21 @@ w4a16_tile_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_const
       // ---------------------------------------------------------------- token rows
       // Thread = one 16-byte piece (8 k) of rows r0, r0 + 4, ...; 16 neighbouring threads copy 256 contiguous bytes.
       // s_rows holds where the tile's rows lie (in 16-byte pieces of x), transposed so that a thread reads four of
-      // its rows at once; the two halves of the pair of warps alternate between two tables.
+      // its rows at once; a warp looks up the rows that it copies itself (r0 = 0, 1 or 2, 3), so that neither warp
+      // ever waits for the other, which may have given up.  Two tables in turn: a lane may still read the last tile's.
       const int th = threadIdx.x - 64, piece = th & 15, r0 = th >> 4;
       const uint4* xv = reinterpret_cast<const uint4*>(P.x) + piece;
       int xs = 0, pending = 0, pslot = 0;                       // groups copied but not yet announced, the oldest's slot
       uint32_t xphase = 0;
       bool ok = true;
       TileWork w = {}, wn = {};
-      int at[2];                                                // rows th and th + 64 of the next tile
+      const int own = 2 * (warp - 2) + (lane & 1);              // this lane looks up rows own + 4 (lane / 2), + 64
+      int at[2];                                                // of the next tile
       auto fetch_rows = [&](const TileWork& t) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int row = t.tok0 + min(th + 64 * h, t.ntok - 1);   // rows past the last repeat it: computed, not stored
-          at[h] = P.perm[row];
+          const int r = own + 4 * (lane >> 1) + 64 * h;
+          at[h] = P.perm[t.tok0 + min(r, t.ntok - 1)];          // rows past the last repeat it: computed, not stored
         }
       };
       if (n_tiles > 0) {
@@ -285,11 +287,9 @@ w4a16_tile_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_const
         w = wn;
         uint32_t* rows = s_rows + (i & 1) * TL_TN;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = th + 64 * h;
-          rows[(r & 3) * (TL_TN / 4) + (r >> 2)] = (uint32_t)(at[h] / P.top_k) * (uint32_t)(Kd / 8);
-        }
-        asm volatile("bar.sync 1, 64;" ::: "memory");
+        for (int h = 0; h < 2; ++h)
+          rows[own * (TL_TN / 4) + (lane >> 1) + 16 * h] = (uint32_t)(at[h] / P.top_k) * (uint32_t)(Kd / 8);
+        __syncwarp();
         if (i + 1 < n_tiles) {
           wn = table.locate(blockIdx.x + (i + 1) * grid);
           fetch_rows(wn);                                       // its latency passes under this tile's copies

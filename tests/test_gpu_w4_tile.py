@@ -1,6 +1,7 @@
 """The W4A16 tile kernel for prefill-size groups (csrc/w4a16_tile.cu): single linears and grouped projections at the
 edges of its tiles (rows 9 to 129 around the 16-row steps and the 128-row tile, columns that end inside a tile or after
-the first of a pair, one and several quantisation groups, empty experts), with contiguous and with gathered rows.
+the first of a pair, one and several quantisation groups, empty experts), with contiguous and with gathered rows, and
+with several tiles to a CTA.
 
 Single linears are held to the fp32 result of the oracle's formula: the kernel multiplies exact integers q - z and adds
 fp32 sums, so only the summation order (about 2^-22 of the sum of magnitudes) and the final rounding to bf16 (2^-9
@@ -21,7 +22,10 @@ DEV = torch.device("cuda", 0)
 
 
 @pytest.mark.parametrize("M,K,N", [(9, 128, 32), (16, 256, 128), (17, 384, 96), (127, 128, 160), (128, 512, 256),
-                                   (129, 256, 384), (300, 128, 4096), (2500, 256, 640)])
+                                   (129, 256, 384), (300, 128, 4096), (2500, 256, 640),
+                                   # two tiles to a CTA: 128 columns each with an odd number of groups; 256 columns
+                                   # with a last pair that ends inside its first or second half or between them
+                                   (4100, 384, 1024), (4100, 384, 2080), (4100, 384, 2176), (4100, 256, 2208)])
 def test_single_linear_at_the_edges_of_the_tiles(M, K, N):
     g = torch.Generator().manual_seed(M + K + N)
     w = torch.randn(K, N, generator=g) * 0.05
@@ -69,6 +73,33 @@ def test_grouped_projections_match_the_oracle(T, H, E, K, I, hot):
         dset = ((down.qweight, down.scales.to(torch.bfloat16), down.qzeros),)
         o32, o64 = (cases.w4_grouped_reference(h.cpu(), dset, off, t) for t in (torch.float32, torch.float64))
         cases.w4_output_bar(o.cpu(), o32, o64)
+    assert status.item() == 0
+
+
+def test_several_tiles_to_a_cta_and_groups_that_share_weights():
+    """More tiles than the CTAs take in two rounds, groups of 0 to over 1000 rows, twice as many groups as weight sets,
+    offsets that start above 0 and end below the rows there are."""
+    T, K, H, E, I = 700, 8, 384, 6, 1024
+    g = torch.Generator().manual_seed(3)
+    gate, up = synthetic._w4_proj(g, E, H, I, 128), synthetic._w4_proj(g, E, H, I, 128)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
+    counts = torch.tensor([5, 0, 1, 16, 17, 127, 128, 129, 1100, 300, 0, 2100, 1650])       # the first: in no group
+    off = counts.cumsum(0).to(torch.int32)
+    lo, hi = int(off[0]), int(off[-1])
+    assert hi < T * K
+    perm = torch.randperm(T * K, generator=g).to(torch.int32).to(DEV)
+    rows = gather_rows(x, perm, K)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    h = w4a16_grouped_swiglu_gather(x, perm, K, dev_set(gate), dev_set(up), off.to(DEV), status=status)
+    plain = w4a16_grouped_swiglu(rows, dev_set(gate), dev_set(up), off.to(DEV))
+    assert torch.equal(plain[lo:hi], h[lo:hi]) and not plain[:lo].any() and not plain[hi:].any()
+    sets = tuple((p.qweight, p.scales.to(torch.bfloat16), p.qzeros) for p in (gate, up))
+    h32, h64 = (cases.w4_grouped_reference(rows.cpu(), sets, off, t) for t in (torch.float32, torch.float64))
+    cases.w4_output_bar(h[lo:hi].cpu(), h32[lo:hi], h64[lo:hi])
+    o = w4a16_grouped_gemm(rows, *dev_set(gate), off.to(DEV))
+    assert not o[:lo].any() and not o[hi:].any()
+    o32, o64 = (cases.w4_grouped_reference(rows.cpu(), sets[:1], off, t) for t in (torch.float32, torch.float64))
+    cases.w4_output_bar(o[lo:hi].cpu(), o32[lo:hi], o64[lo:hi])
     assert status.item() == 0
 
 
