@@ -48,7 +48,10 @@ constexpr int TL_SMEM = TL_NX * TL_XSLOT + TL_NW * TL_WSLOT + TL_BARS + TL_ROWS 
 constexpr int TL_THREADS = 640;
 constexpr int TL_A_COL = 256;                    // TMEM: two accumulators of 128 columns, then four A buffers of 64
 
-enum TileMode { TILE_SWIGLU, TILE_WIDE, TILE_NARROW };
+// SWIGLU_EXACT: SWIGLU with expf and a true quotient, for the calls that had them on the cp.async kernel (the stream
+// kernel's SwiGLU has the approximations).
+enum TileMode { TILE_SWIGLU, TILE_SWIGLU_EXACT, TILE_WIDE, TILE_NARROW };
+__host__ __device__ constexpr bool tile_swiglu(int mode) { return mode == TILE_SWIGLU || mode == TILE_SWIGLU_EXACT; }
 
 struct TileProj {
   const __nv_bfloat16* sc;                       // [period, G, N]
@@ -179,13 +182,13 @@ w4a16_tile_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_const
         for (int u = 0; u < U; ++u) {
           const int g = NSUB == 2 ? u >> 1 : u, sub = NSUB == 2 ? u & 1 : 0;
           const int n0 = w.n0 + (MODE == TILE_WIDE ? sub * TL_M : 0);
-          const TileProj& p = (MODE == TILE_SWIGLU && sub) ? P.p1 : P.p0;
+          const TileProj& p = (tile_swiglu(MODE) && sub) ? P.p1 : P.p0;
           ok = mbar_wait(wempty(slot), phase ^ 1u, abort_flag, P.d_status);
           if (!ok) break;
           const uint32_t dst = wring + slot * TL_WSLOT;
           const int cols = max(0, min(TL_M, N - n0));           // a multiple of 32
           mbar_expect_tx(wfull(slot), (uint32_t)(TL_WORDS + 2 * cols + cols / 2));
-          tma_load_2d(dst, (MODE == TILE_SWIGLU && sub) ? &map_w1 : &map_w0, wfull(slot), n0, (we * G + g) * (TL_K / 8));
+          tma_load_2d(dst, (tile_swiglu(MODE) && sub) ? &map_w1 : &map_w0, wfull(slot), n0, (we * G + g) * (TL_K / 8));
           if (cols > 0) {
             const size_t row = (size_t)we * G + g;
             bulk_load(dst + TL_SC_OFF, p.sc + row * N + n0, 2 * cols, wfull(slot));
@@ -455,9 +458,12 @@ w4a16_tile_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_const
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             float2 v = unpack2(master[s][c][j]);
-            if (MODE == TILE_SWIGLU) {
+            if (tile_swiglu(MODE)) {
               const float2 u = unpack2(master[NSUB - 1][c][j]);
-              v = make_float2(swiglu_fast(v.x, u.x), swiglu_fast(v.y, u.y));
+              if (MODE == TILE_SWIGLU_EXACT)
+                v = make_float2(swiglu_rounded<__nv_bfloat16>(v.x, u.x), swiglu_rounded<__nv_bfloat16>(v.y, u.y));
+              else
+                v = make_float2(swiglu_fast(v.x, u.x), swiglu_fast(v.y, u.y));
             }
             const float other = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
             const __nv_bfloat162 r = odd ? __floats2bfloat162_rn(other, v.y) : __floats2bfloat162_rn(v.x, other);
@@ -510,6 +516,8 @@ bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t 
          period * (Kd / 8) < ((int64_t)1 << 31) && (S / 16 + E) * (N / 32) < ((int64_t)1 << 30);
 }
 
+bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
+
 // x: rows in natural k order, [S, Kd] or (perm) [x_rows, Kd] gathered by row = perm[p] / top_k.
 int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k, const int32_t* qw0, const void* sc0,
                const int32_t* qz0, const int32_t* qw1, const void* sc1, const int32_t* qz1, bool swiglu,
@@ -554,8 +562,12 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
     cudaFuncSetAttribute(w4a16_tile_kernel<MODE, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM);    \
     w4a16_tile_kernel<MODE, GATHER><<<grid, TL_THREADS, TL_SMEM, st>>>(map0, map1, mapx, P);                        \
   } while (0)
-  if (swiglu && perm != nullptr) MQ_TILE_LAUNCH(TILE_SWIGLU, true);
-  else if (perm != nullptr) return MQ_ERR_UNSUPPORTED_SHAPE;
+  // no coarser a SwiGLU than without this kernel: the stream kernel takes 32 rows or more of up to 384 groups
+  const bool exact = swiglu && (S < 32 || !w4a16_stream_covers(S, E, period, N, Kd, 128));
+  if (perm != nullptr && !swiglu) return MQ_ERR_UNSUPPORTED_SHAPE;
+  if (exact && perm != nullptr) MQ_TILE_LAUNCH(TILE_SWIGLU_EXACT, true);
+  else if (exact) MQ_TILE_LAUNCH(TILE_SWIGLU_EXACT, false);
+  else if (swiglu && perm != nullptr) MQ_TILE_LAUNCH(TILE_SWIGLU, true);
   else if (swiglu) MQ_TILE_LAUNCH(TILE_SWIGLU, false);
   else if (wide) MQ_TILE_LAUNCH(TILE_WIDE, false);
   else MQ_TILE_LAUNCH(TILE_NARROW, false);

@@ -103,6 +103,23 @@ def test_several_tiles_to_a_cta_and_groups_that_share_weights():
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("counts,E", [((9, 11, 10), 3), ([8, 9, 8] * 133 + [30], 8)])
+def test_swiglu_keeps_the_exact_quotient_where_the_stream_kernel_did_not_run(counts, E):
+    """Fewer than 32 rows, and more than 384 groups: silu with expf and a true quotient, i.e. torch's own silu of the
+    bf16 gate, bit for bit (an approximation falls to the other bf16 neighbour once in about 2^11 elements)."""
+    H, I = 256, 2048 if E == 3 else 256
+    g = torch.Generator().manual_seed(E)
+    gate, up = (dev_set(synthetic._w4_proj(g, E, H, I, 128)) for _ in range(2))
+    off = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    S = int(off[-1])
+    assert S > 8 * len(counts)
+    x = (torch.randn(S, H, generator=g) * 0.3).to(torch.bfloat16).to(DEV)
+    want = torch.nn.functional.silu(w4a16_grouped_gemm(x, *gate, off)) * w4a16_grouped_gemm(x, *up, off)
+    assert torch.equal(w4a16_grouped_swiglu(x, gate, up, off), want)
+    perm = torch.arange(S, dtype=torch.int32, device=DEV)
+    assert torch.equal(w4a16_grouped_swiglu_gather(x, perm, 1, gate, up, off), want)
+
+
 def test_gather_entry_point_rejects_what_the_kernel_does_not_cover():
     x = torch.zeros(4, 128, dtype=torch.bfloat16, device=DEV)
     w = tuple(t.to(DEV) for t in (torch.zeros(1, 16, 40, dtype=torch.int32), torch.zeros(1, 1, 40, dtype=torch.bfloat16),
