@@ -440,19 +440,45 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
 }  // namespace
 }  // namespace mq
 
+extern "C" int mq_w4a16_grouped_gemm_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
+                                        const int32_t* offsets, int64_t S, int64_t E, int64_t weight_period, int64_t N,
+                                        int64_t Kd, int64_t group_size, void* out, int32_t* d_status, void* stream) {
+  mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
+  return mq::launch_w4(x, p, p, false, offsets, S, E, weight_period, N, Kd, group_size, out,
+                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status);
+}
+
 extern "C" int mq_w4a16_grouped_gemm(const void* x, const int32_t* qweight, const void* scales,
                                      const int32_t* qzeros, const int32_t* offsets,
                                      int64_t S, int64_t E, int64_t weight_period, int64_t N, int64_t Kd,
                                      int64_t group_size, void* out, void* stream) {
+  return mq_w4a16_grouped_gemm_ex(x, qweight, scales, qzeros, offsets, S, E, weight_period, N, Kd, group_size, out, nullptr,
+                                  stream);
+}
+
+extern "C" int mq_w4a16_linear_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
+                                  int64_t M, int64_t N, int64_t Kd, int64_t group_size, void* out, int32_t* d_status,
+                                  void* stream) {
   mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
-  return mq::launch_w4(x, p, p, false, offsets, S, E, weight_period, N, Kd, group_size, out,
-                       reinterpret_cast<cudaStream_t>(stream));
+  return mq::launch_w4(x, p, p, false, nullptr, M, 1, 1, N, Kd, group_size, out, reinterpret_cast<cudaStream_t>(stream),
+                       nullptr, 1, d_status);
 }
 
 extern "C" int mq_w4a16_linear(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros, int64_t M,
                                int64_t N, int64_t Kd, int64_t group_size, void* out, void* stream) {
-  mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
-  return mq::launch_w4(x, p, p, false, nullptr, M, 1, 1, N, Kd, group_size, out, reinterpret_cast<cudaStream_t>(stream));
+  return mq_w4a16_linear_ex(x, qweight, scales, qzeros, M, N, Kd, group_size, out, nullptr, stream);
+}
+
+extern "C" int mq_w4a16_grouped_swiglu_ex(const void* x,
+                                          const int32_t* qweight_gate, const void* scales_gate,
+                                          const int32_t* qzeros_gate, const int32_t* qweight_up, const void* scales_up,
+                                          const int32_t* qzeros_up, const int32_t* offsets,
+                                          int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H,
+                                          int64_t group_size, void* h, int32_t* d_status, void* stream) {
+  mq::W4Proj p0{qweight_gate, reinterpret_cast<const __nv_bfloat16*>(scales_gate), qzeros_gate};
+  mq::W4Proj p1{qweight_up, reinterpret_cast<const __nv_bfloat16*>(scales_up), qzeros_up};
+  return mq::launch_w4(x, p0, p1, true, offsets, S, E, weight_period, I, H, group_size, h,
+                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status);
 }
 
 extern "C" int mq_w4a16_grouped_swiglu(const void* x,
@@ -461,10 +487,8 @@ extern "C" int mq_w4a16_grouped_swiglu(const void* x,
                                        const int32_t* offsets,
                                        int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H,
                                        int64_t group_size, void* h, void* stream) {
-  mq::W4Proj pg{qweight_gate, reinterpret_cast<const __nv_bfloat16*>(scales_gate), qzeros_gate};
-  mq::W4Proj pu{qweight_up, reinterpret_cast<const __nv_bfloat16*>(scales_up), qzeros_up};
-  return mq::launch_w4(x, pg, pu, true, offsets, S, E, weight_period, I, H, group_size, h,
-                       reinterpret_cast<cudaStream_t>(stream));
+  return mq_w4a16_grouped_swiglu_ex(x, qweight_gate, scales_gate, qzeros_gate, qweight_up, scales_up, qzeros_up, offsets, S,
+                                    E, weight_period, I, H, group_size, h, nullptr, stream);
 }
 
 extern "C" int mq_w4a16_grouped_swiglu_gather(const void* x, const int32_t* perm,

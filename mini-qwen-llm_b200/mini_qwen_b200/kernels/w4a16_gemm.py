@@ -41,9 +41,11 @@ def _check_w4(x, qweight, scales, qzeros, group_size, E, prepared_f16=False):
 
 
 def w4a16_grouped_gemm(x, qweight, scales, qzeros, expert_offsets, group_size: int = 128,
-                       zero_init: bool = True, out: torch.Tensor | None = None) -> torch.Tensor:
+                       zero_init: bool = True, out: torch.Tensor | None = None,
+                       status: torch.Tensor | None = None) -> torch.Tensor:
     """Rows ``offsets[e]:offsets[e+1]`` of x times the dequantised weight of expert e.
-    qweight [E, K/8, N], scales [E, K/g, N], qzeros [E, K/g, N/8], offsets int32 [E+1]."""
+    qweight [E, K/8, N], scales [E, K/g, N], qzeros [E, K/g, N/8], offsets int32 [E+1].  ``status`` (int32 [1],
+    optional) receives device-side error bits (a bounded wait that ran out)."""
     E = qweight.shape[0]
     K, N = _check_w4(x, qweight, scales, qzeros, group_size, E)
     expert_offsets = _offsets32(expert_offsets)
@@ -54,16 +56,18 @@ def w4a16_grouped_gemm(x, qweight, scales, qzeros, expert_offsets, group_size: i
     if out is None:
         out = (torch.zeros if zero_init else torch.empty)(S, N, dtype=torch.bfloat16, device=x.device)
     assert out.is_contiguous() and tuple(out.shape) == (S, N) and out.dtype == torch.bfloat16
-    rc = _cabi.load().mq_w4a16_grouped_gemm(_cabi.ptr(x), _cabi.ptr(qweight), _cabi.ptr(scales), _cabi.ptr(qzeros),
-                                            _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(out),
-                                            _cabi.stream_ptr(x.device))
+    rc = _cabi.load().mq_w4a16_grouped_gemm_ex(_cabi.ptr(x), _cabi.ptr(qweight), _cabi.ptr(scales), _cabi.ptr(qzeros),
+                                               _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(out),
+                                               _cabi.ptr(status), _cabi.stream_ptr(x.device))
     _cabi.check(rc, "mq_w4a16_grouped_gemm")
     _cabi.count_launches(1 if S else 0)
     return out
 
 
-def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zero_init: bool = True) -> torch.Tensor:
-    """Fused gate/up W4A16 projections + SwiGLU; gate and up are (qweight, scales, qzeros) stacks."""
+def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zero_init: bool = True,
+                         status: torch.Tensor | None = None) -> torch.Tensor:
+    """Fused gate/up W4A16 projections + SwiGLU; gate and up are (qweight, scales, qzeros) stacks; ``status`` as in
+    :func:`w4a16_grouped_gemm`."""
     E = gate[0].shape[0]
     K, N = _check_w4(x, *gate, group_size, E)
     _check_w4(x, *up, group_size, E)
@@ -73,10 +77,10 @@ def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zer
     x = x.contiguous()
     S = x.shape[0]
     h = (torch.zeros if zero_init else torch.empty)(S, N, dtype=torch.bfloat16, device=x.device)
-    rc = _cabi.load().mq_w4a16_grouped_swiglu(_cabi.ptr(x), _cabi.ptr(gate[0]), _cabi.ptr(gate[1]), _cabi.ptr(gate[2]),
-                                              _cabi.ptr(up[0]), _cabi.ptr(up[1]), _cabi.ptr(up[2]),
-                                              _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(h),
-                                              _cabi.stream_ptr(x.device))
+    rc = _cabi.load().mq_w4a16_grouped_swiglu_ex(
+        _cabi.ptr(x), _cabi.ptr(gate[0]), _cabi.ptr(gate[1]), _cabi.ptr(gate[2]), _cabi.ptr(up[0]), _cabi.ptr(up[1]),
+        _cabi.ptr(up[2]), _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(h), _cabi.ptr(status),
+        _cabi.stream_ptr(x.device))
     _cabi.check(rc, "mq_w4a16_grouped_swiglu")
     _cabi.count_launches(1 if S else 0)
     return h
@@ -116,8 +120,10 @@ def w4a16_gemm(
     scales: torch.Tensor,
     qzeros: torch.Tensor,
     group_size: int = 128,
+    status: torch.Tensor | None = None,
 ) -> torch.Tensor:
-    """``x @ dequant(qweight)`` with ``W[k,n] = (q[k,n] - z[k//g,n]) * s[k//g,n]``; returns bf16 [M, N]."""
+    """``x @ dequant(qweight)`` with ``W[k,n] = (q[k,n] - z[k//g,n]) * s[k//g,n]``; returns bf16 [M, N].
+    ``status`` as in :func:`w4a16_grouped_gemm`."""
     assert x.dim() == 2 and qweight.dim() == 2
     if not (qweight.is_contiguous() and scales.is_contiguous() and qzeros.is_contiguous()):
         qweight, scales, qzeros = qweight.contiguous(), scales.contiguous(), qzeros.contiguous()
@@ -126,8 +132,9 @@ def w4a16_gemm(
         x = x.contiguous()
     M = x.shape[0]
     out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-    rc = _cabi.load().mq_w4a16_linear(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), M, N, K,
-                                      group_size, out.data_ptr(), _cabi.stream_ptr(x.get_device()))
+    rc = _cabi.load().mq_w4a16_linear_ex(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), M, N, K,
+                                         group_size, out.data_ptr(), None if status is None else status.data_ptr(),
+                                         _cabi.stream_ptr(x.get_device()))
     if rc:
         _cabi.check(rc, "mq_w4a16_linear")
     _cabi.count_launches(1 if M else 0)

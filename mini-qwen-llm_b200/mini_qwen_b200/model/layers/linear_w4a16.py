@@ -18,6 +18,8 @@ class LinearW4A16(nn.Module):
     ``qzeros`` int32 [K/g, N/8] (8 values per word along N).
     """
 
+    _status = None     # device status word, allocated by the first call of more than eight rows
+
     def __init__(self, in_features: int, out_features: int, group_size: int = 128):
         super().__init__()
         self.in_features = in_features
@@ -34,10 +36,19 @@ class LinearW4A16(nn.Module):
             qweight, scales, qzeros = buf["qweight"], buf["scales"], buf["qzeros"]
         except KeyError:                     # not kept there: parametrizations, buffers turned into parameters
             qweight, scales, qzeros = self.qweight, self.scales, self.qzeros
-        if x.dim() == 2 and x.shape[1] == self.in_features:
-            return w4a16_gemm(x, qweight, scales, qzeros, self.group_size)
-        y = w4a16_gemm(x.reshape(-1, self.in_features), qweight, scales, qzeros, self.group_size)
-        return y.reshape(*x.shape[:-1], self.out_features)
+        rows = x if x.dim() == 2 and x.shape[1] == self.in_features else x.reshape(-1, self.in_features)
+        status = None
+        if rows.shape[0] > 8 and rows.is_cuda:     # up to eight rows: a kernel without bounded waits
+            status = self._status
+            if status is None or status.device != rows.device:
+                status = self._status = torch.zeros(1, dtype=torch.int32, device=rows.device)
+        y = w4a16_gemm(rows, qweight, scales, qzeros, self.group_size, status)
+        return y if rows is x else y.reshape(*x.shape[:-1], self.out_features)
+
+    def check_status(self) -> None:
+        """Raises if a kernel of this layer reported a device-side error (synchronises)."""
+        if self._status is not None and int(self._status.item()) & 1:
+            raise RuntimeError("a bounded wait expired inside a W4A16 kernel; the last output is invalid")
 
     @classmethod
     def from_float(cls, linear: nn.Linear, group_size: int = 128) -> "LinearW4A16":

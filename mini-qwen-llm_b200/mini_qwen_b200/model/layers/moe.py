@@ -409,7 +409,7 @@ class Qwen3MoEBlock(nn.Module):
             h = run("grouped_swiglu", w4a16_grouped_swiglu_gather, x2d, perm, K, st["gate_proj"], st["up_proj"], off32,
                     st["group_size"], status=status)
             out_perm = run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off32, st["group_size"],
-                           zero_init=False)
+                           zero_init=False, status=status)
             return run("unpermute_combine", unpermute_combine, out_perm, weights, inv, T, K, residual=res).reshape(shape)
         if self.ep_size == 1 and st["w4"] and self._w4_stream(st):
             # decode path: one preparation launch replaces the row gather, the gate/up kernel then needs no byte
@@ -425,7 +425,7 @@ class Qwen3MoEBlock(nn.Module):
                 h = run("grouped_swiglu", w4a16_stream_swiglu, xp, xs, st["gate_proj"], st["up_proj"], off32,
                         st["group_size"], shuffle_out=False, status=status)
             out_perm = run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off32, st["group_size"],
-                           zero_init=False)
+                           zero_init=False, status=status)
             return run("unpermute_combine", unpermute_combine, out_perm, weights, inv, T, K, residual=res).reshape(shape)
         if self.ep_size == 1 and st["w4"] and self._w4_tc(st, T * K):
             # decode-size groups: weights dequantised into tensor memory, activations prepared once
@@ -465,12 +465,12 @@ class Qwen3MoEBlock(nn.Module):
         """Grouped gate/up + SwiGLU and down projection over rows grouped by `off32`."""
         run = self._stage
         # the groups of a routing cover every row that is read later, so no output needs a zero fill
+        status = self._status_word(rows.device)
         if st["w4"]:
             h = run("grouped_swiglu", w4a16_grouped_swiglu, rows, st["gate_proj"], st["up_proj"], off32,
-                    st["group_size"], zero_init=False)
+                    st["group_size"], zero_init=False, status=status)
             return run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off32, st["group_size"],
-                       zero_init=False, out=out)
-        status = self._status_word(rows.device)
+                       zero_init=False, out=out, status=status)
         h = run("grouped_swiglu", moe_grouped_swiglu, rows, st["w13"], off32, zero_init=False, status=status)
         return run("grouped_down", moe_grouped_gemm, h, st["w2"], off32, zero_init=False, out=out, status=status)
 
@@ -566,7 +566,7 @@ class Qwen3MoEBlock(nn.Module):
         h = run("grouped_swiglu", w4a16_stream_swiglu, xp_tok, xs_tok, st["gate_proj"], st["up_proj"], off_local,
                 st["group_size"], shuffle_out=False, status=status, perm=perm, top_k=K)
         out_perm = run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off_local, st["group_size"],
-                       zero_init=False)
+                       zero_init=False, status=status)
         run("send_partials", peer.send_partials, out_perm, weights, ids32, inv, T, K, el)   # barrier inside
         return run("sum_partials", peer.sum_partials, T, res)
 

@@ -10,11 +10,12 @@ import pytest
 import torch
 
 import cases
-from mini_qwen_b200 import _cabi, synthetic
+from mini_qwen_b200 import Qwen3MoEConfig, _cabi, synthetic
 from mini_qwen_b200.kernels import moe_permute_plan
 from mini_qwen_b200.kernels.moe_permute import gather_rows
 from mini_qwen_b200.kernels.w4a16_gemm import (w4a16_gemm, w4a16_grouped_gemm, w4a16_grouped_swiglu,
                                                w4a16_grouped_swiglu_gather)
+from mini_qwen_b200.model.layers import LinearW4A16, Qwen3MoEBlock
 from oracle import moe_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -128,3 +129,48 @@ def test_gather_entry_point_rejects_what_the_kernel_does_not_cover():
     off = torch.tensor([0, 4], dtype=torch.int32, device=DEV)
     with pytest.raises(ValueError):
         w4a16_grouped_swiglu_gather(x, perm, 1, w, w, off)                 # 40 columns: not a multiple of 32
+
+
+class Recorder:
+    """The library, with the arguments of every call kept."""
+
+    def __init__(self, lib):
+        self.lib, self.calls = lib, []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, args))
+            return getattr(self.lib, name)(*args)
+        return call
+
+
+def test_every_launch_of_the_kernel_has_a_status_word(monkeypatch):
+    """The kernel leaves part of its result unwritten when a bounded wait runs out; check_status() must be able to say
+    so.  (No wait is made to run out here: the word is set by hand.)"""
+    spy = Recorder(_cabi.load())
+    monkeypatch.setattr(_cabi, "load", lambda: spy)
+    lin = LinearW4A16(256, 128).to(DEV)
+    x = torch.randn(200, 256, device=DEV).to(torch.bfloat16)
+    lin(x[:8])
+    lin.check_status()
+    lin(x)
+    lin(x.reshape(2, 100, 256))
+    launches = [a for n, a in spy.calls if n == "mq_w4a16_linear_ex"]
+    assert [a[-2] for a in launches] == [None, lin._status.data_ptr(), lin._status.data_ptr()]
+    lin.check_status()
+    lin._status.fill_(1)
+    with pytest.raises(RuntimeError):
+        lin.check_status()
+    assert set(lin.state_dict()) == {"qweight", "scales", "qzeros"}
+
+    cfg = Qwen3MoEConfig(hidden_size=256, intermediate_size=128, num_experts=8, num_experts_per_tok=2)
+    blk = Qwen3MoEBlock.from_stacked_w4(cfg, torch.randn(8, 256, device=DEV).to(torch.bfloat16),
+                                        *synthetic.w4a16_stacks_on_device(DEV, 3, 8, 256, 128))
+    for kernel in ("stream", "mma"):
+        spy.calls.clear()
+        blk.w4_kernel = kernel
+        blk._forward_staged(x)
+        word = blk._status.data_ptr()
+        seen = [n for n, a in spy.calls if n.startswith("mq_w4a16_grouped") and word in a]
+        assert len(seen) == 2 and all(word in a for n, a in spy.calls if n.startswith("mq_w4a16_grouped")), spy.calls
+    blk.check_status()

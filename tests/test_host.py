@@ -284,3 +284,19 @@ def test_finalize_drops_the_description_of_the_old_stacks(quantised):
     assert blk._native is not None
     blk.finalize()
     assert blk._native is None
+
+
+def test_the_block_call_hands_its_status_word_to_every_kernel_that_has_bounded_waits():
+    """In csrc/block.cu: each library call that takes a status word is given the caller's, and none is made in a form
+    without one (mq_x where mq_x_ex has one)."""
+    header = open(os.path.join(ROOT, "include", "mqmoe.h")).read()
+    prototypes = dict(re.findall(r"\bint (mq_[a-z0-9_]+)\(([^;]*)\);", header))
+    with_status = {n for n, args in prototypes.items() if "d_status" in args}
+    without = {n for n in prototypes if n + "_ex" in with_status}
+    source = open(os.path.join(ROOT, "mini-qwen-llm_b200", "csrc", "block.cu")).read()
+    source = source[source.index('extern "C" int mq_moe_forward('):]
+    calls = re.findall(r"MQ_BLOCK_STEP\((mq_[a-z0-9_]+)\((.*?)\)\);", source, flags=re.S)
+    named = {n for n, _ in calls}
+    assert {"mq_w4a16_grouped_gemm_ex", "mq_grouped_gemm"} <= named and not named & without
+    for name, args in calls:
+        assert name not in with_status or "d_status" in args, name
