@@ -33,8 +33,10 @@ BlockPlan plan_of(const mq_moe_layer& L, int64_t T) {
   // decode batches: logits, top-k, plan (and the W4A16 activation preparation) in one launch
   p.small = T <= 64 && E <= 256 && K <= 32 && S <= 2048;
   if (p.w4) {
-    // more than eight rows per expert on average: the tile kernel (the rule of the W4A16 dispatch)
-    p.tile = S > 8 * E && w4a16_tile_covers(S, E, E, I, H, L.group_size) && T * (H / 8) < ((int64_t)1 << 32);
+    // more than eight rows per expert on average: the tile kernel (the rule of the W4A16 dispatch), whose bulk copies
+    // want the zero points 16-byte aligned; the other kernels read them word by word
+    p.tile = S > 8 * E && w4a16_tile_covers(S, E, E, I, H, L.group_size) && T * (H / 8) < ((int64_t)1 << 32) &&
+             aligned16(L.gate[2]) && aligned16(L.up[2]);
     p.stream = !p.tile && H <= 4096 && w4a16_stream_covers(S, E, E, I, H, L.group_size);
     p.prepared = p.stream && p.small && T <= E;
     p.gather_in_kernel = p.tile || p.stream;

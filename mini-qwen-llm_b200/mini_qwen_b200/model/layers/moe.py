@@ -476,8 +476,10 @@ class Qwen3MoEBlock(nn.Module):
 
     def _w4_tile(self, st, slots: int) -> bool:
         """Whether both projections run on the tensor-core tile kernel: more than eight slots per expert on average
-        (the rule of the library's own dispatch) and shapes it covers."""
+        (the rule of the library's own dispatch) and tensors it covers."""
         if self.w4_kernel != "stream" or slots <= 8 * self.num_local_experts:
+            return False
+        if any(st[p][2].data_ptr() % 16 for p in ("gate_proj", "up_proj")):
             return False
         qw = st["gate_proj"][0]
         return w4a16_gather_supported(qw.shape[1] * 8, qw.shape[2], st["group_size"], self.num_local_experts)

@@ -70,3 +70,26 @@ def test_description_follows_the_layer():
         blk(x, residual=x[:1])
     with pytest.raises(ValueError):
         blk(x.cpu())
+
+
+def test_zero_points_off_the_16_byte_grid():
+    """Stacks that are views into a flat buffer at a multiple of four bytes: accepted at every batch size, with the
+    results of aligned ones (another kernel's order of the fp32 sums, so within a few bf16 roundings)."""
+    E, K, H, I = 8, 2, 256, 128
+    cfg = Qwen3MoEConfig(hidden_size=H, intermediate_size=I, num_experts=E, num_experts_per_tok=K)
+    router = torch.randn(E, H, device=DEV).to(torch.bfloat16)
+    stacks = synthetic.w4a16_stacks_on_device(DEV, 7, E, H, I)
+
+    def view(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        flat[1:] = t.reshape(-1)
+        return flat[1:].view(t.shape)
+    blk = Qwen3MoEBlock.from_stacked_w4(cfg, router, *stacks)
+    off = Qwen3MoEBlock.from_stacked_w4(cfg, router, *[(qw, sc, view(qz)) for qw, sc, qz in stacks])
+    for T in (3, 64, 65, 400):
+        x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+        out = off(x)
+        assert torch.equal(out, off._forward_staged(x))
+        want = blk(x).float()
+        assert float((out.float() - want).norm() / want.norm()) < 1e-2
+    off.check_status()

@@ -300,3 +300,30 @@ def test_the_block_call_hands_its_status_word_to_every_kernel_that_has_bounded_w
     assert {"mq_w4a16_grouped_gemm_ex", "mq_grouped_gemm"} <= named and not named & without
     for name, args in calls:
         assert name not in with_status or "d_status" in args, name
+
+
+def test_zero_points_off_the_16_byte_grid_keep_a_layer_off_the_tile_kernel():
+    """Views into a flat checkpoint buffer: the tile kernel copies zero points in bulk and refuses them, the others read
+    them word by word.  The stream kernel's prepared rows show in the workspace."""
+    lib = _cabi.load()
+    L = _cabi.MoELayer(hidden=256, inter=128, experts=8, top_k=2, group_size=128, dtype=_cabi.MQ_BF16,
+                       router_dtype=_cabi.MQ_BF16, renormalize=1)
+    for name in ("gate", "up", "down"):
+        for i in range(3):
+            getattr(L, name)[i] = 4096
+    T, rows = 200, 400
+    tile = lib.mq_moe_forward_workspace_bytes(ctypes.addressof(L), T)
+    L.down[2] = 4100
+    assert lib.mq_moe_forward_workspace_bytes(ctypes.addressof(L), T) == tile
+    for name in ("gate", "up"):
+        getattr(L, name)[2] = 4100
+        assert lib.mq_moe_forward_workspace_bytes(ctypes.addressof(L), T) >= tile + rows * 256 * 2
+        getattr(L, name)[2] = 4096
+    blk = _small_block(True)
+    flat = torch.zeros(257, dtype=torch.int32)
+    at = (-flat.data_ptr() // 4) % 4
+    for off, want in ((at, True), (at + 1, False)):
+        st = {"gate_proj": (torch.zeros(2, 16, 32), None, flat[off:]), "up_proj": (None, None, flat[at:]), "group_size": 128}
+        assert blk._w4_tile(st, 1000) is want
+        st["gate_proj"], st["up_proj"] = (st["gate_proj"][0], None, flat[at:]), (None, None, flat[off:])
+        assert blk._w4_tile(st, 1000) is want
