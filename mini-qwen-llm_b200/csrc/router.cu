@@ -458,11 +458,11 @@ __device__ void route_prepare_row(const __nv_bfloat16* __restrict__ x_row, int H
   }
 }
 
-// ---- the same for batches of more than 16 tokens, laid out by TOKEN: CTA (eg, t) forms the logits of experts
+// ---- the same laid out by TOKEN, for batches of more than 16 tokens and for small fp32 layers: CTA (eg, t) forms the logits of experts
 // [32 eg, 32 eg + 32) for token t (a warp takes four experts; a lane keeps its pieces of the token's row in
 // registers; all loads of a lane are independent: one round trip), the CTA that arrives last on token t's counter
 // does that token's softmax and top-k (one warp), and the CTA that finishes the last token makes the plan.  The
-// selection of the tokens thus runs on as many SMs as there are tokens instead of on one.  16-bit x and w only.
+// selection of the tokens thus runs on as many SMs as there are tokens instead of on one.
 constexpr int RTK_THREADS = 256;
 constexpr int RTK_HEADER_INTS = 128;                  // workspace header: counter of the narrow kernel, all-tokens
                                                       // counter, one counter per token (64)
@@ -492,18 +492,38 @@ route_tokens_kernel(const void* __restrict__ xv_, int xdt, const void* __restric
     const int e0 = eg * 32 + warp;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (F32) {
-      for (int pc = lane; pc < pieces; pc += 32) {
-        float a[8], b[4][8];
-        load8(xv_, xdt, (size_t)t * H + 8 * pc, a);
+      // Every piece's eight products are added up by themselves and the pieces' sums in pairs, as deep a tree as the
+      // expert-major kernel's (eight products a thread, then the threads): one chain of H / 32 products a lane would
+      // add up fp32 logits less exactly.
+      for (int p0 = 0; p0 < pieces; p0 += 32 * MAXP) {
+        float part[MAXP][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (e0 + 8 * j < E) load8(wv_, wdt, (size_t)(e0 + 8 * j) * H + 8 * pc, b[j]);
+        for (int i = 0; i < MAXP; ++i) {
+          const int pc = p0 + lane + 32 * i;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (e0 + 8 * j < E) {
+          for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
+          if (pc < pieces) {
+            float a[8], b[4][8];
+            load8(xv_, xdt, (size_t)t * H + 8 * pc, a);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc[j] = fmaf(a[q], b[j][q], acc[j]);
+            for (int j = 0; j < 4; ++j)
+              if (e0 + 8 * j < E) load8(wv_, wdt, (size_t)(e0 + 8 * j) * H + 8 * pc, b[j]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (e0 + 8 * j < E) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) part[i][j] = fmaf(a[q], b[j][q], part[i][j]);
+              }
           }
+        }
+#pragma unroll
+        for (int d = 1; d < MAXP; d *= 2)
+#pragma unroll
+          for (int i = 0; i < MAXP; i += 2 * d)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] += part[i + d][j];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] += part[0][j];
       }
     } else {
       const uint16_t* xr = reinterpret_cast<const uint16_t*>(xv_) + (size_t)t * H;
@@ -870,6 +890,19 @@ extern "C" size_t mq_route_small_workspace_bytes(int64_t T, int64_t E) {
   return (size_t)T * (size_t)E * sizeof(float) + 512;       // a header of counters, then the logits
 }
 
+namespace mq {
+namespace {
+// us, expert- against token-major (runs differ by 5 %): 4 tokens of 256, 8 experts 7.4 | 6.8; 16 of 512, 32 experts
+// 8.4 | 7.4; 17 of 1024, 64 experts 10.7 | 9.7; 24 of 2048, 64 experts 12.7 | 11.5; 64 of 256, 8 experts 17 | 7.  But 2 of
+// 512, 8 experts 6.3 | 6.8; 16 of 1024, 32 experts 7.9 | 8.3; 4 of 2048, 32 experts 6.5 | 9.2; 17 of 2048, 64 experts
+// 10.9 | 11.5.
+bool fp32_by_token(int64_t T, int64_t H, int64_t E) {
+  if (T <= 16) return E <= 32 && T >= 4 && H <= 512;
+  return H <= 1024 || (H <= 2048 && T >= 24);
+}
+}  // namespace
+}  // namespace mq
+
 extern "C" int mq_route_small(const void* x, int x_dtype, const void* w, int w_dtype, const float* bias,
                               int64_t T, int64_t H, int64_t E, int64_t K, int renormalize,
                               void* workspace, size_t workspace_bytes, int64_t* ids64, int32_t* ids32,
@@ -898,10 +931,13 @@ extern "C" int mq_route_small(const void* x, int x_dtype, const void* w, int w_d
   int* counter = reinterpret_cast<int*>(workspace);
   float* logits = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + RTK_HEADER_INTS * sizeof(int));
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (vec_ok && (T > 16 || E <= 32)) {
-    // The token-major kernel (selection on as many SMs as there are tokens) where one CTA has fewer warps than there
-    // are tokens, or where few experts leave the expert-major kernel with a handful of CTAs (fp32 layer, 8 experts, 64
-    // tokens: 17.3 us there, one CTA per expert).
+  // The token-major kernel (selection on as many SMs as there are tokens) where one CTA has fewer warps than there are
+  // tokens.  Up to 16 tokens its CTAs read the whole router matrix each where the expert-major kernel has a CTA per
+  // expert, and its two levels of counters cost more than the parallel selection gains (16-bit, us, expert- against
+  // token-major at 1, 4, 16 tokens of 1024: 5.8 6.0 6.6 | 6.8 6.9 6.9 with 8 experts, 5.9 6.0 7.4 | 7.6 7.3 8.1 with 16,
+  // 6.3 6.4 6.4 | 9.3 8.9 9.0 with 32).  fp32 rows, which the expert-major kernel reads piece by piece: fp32_by_token.
+  const bool f32 = x_dtype == MQ_F32 || w_dtype == MQ_F32;
+  if (vec_ok && (f32 ? fp32_by_token(T, H, E) : T > 16)) {
     const size_t smem_t = (size_t)E * 8 + (size_t)E * 4 + (size_t)T * K * 4 + (size_t)E * 4;
     const dim3 grid((unsigned)((E + 31) / 32), (unsigned)T);
 #define MQ_RTK_LAUNCH(EPL)                                                                                       \
