@@ -38,7 +38,8 @@ constexpr int P_BOX_BYTES = P_BOX * PK * 2;
 constexpr int P_EPI = 8, P_GATHER = 4;           // warps
 constexpr int P_STG = 32 * 64;                   // staged output rows of an epilogue warp
 constexpr int P_MAX_E = 1024;
-constexpr int P_TABLE = 2 * (P_MAX_E + 1) * 4;
+constexpr int P_SORT_E = 256;                    // most groups that are put in order of size
+constexpr int P_TABLE = (2 * (P_MAX_E + 1) + P_SORT_E) * 4;
 constexpr int P_SMEM = 1024 + P_NST * P_STAGE + P_EPI * P_STG + 256 + ((P_TABLE + 15) & ~15);
 static_assert(P_SMEM <= 232448, "shared memory of a CTA");
 
@@ -152,9 +153,15 @@ struct PairTile {
   int n0, n1;                                    // MMA N of the token chunks (multiples of 32; n1 = 0: one chunk)
 };
 
+// Tiles are dealt out in the groups' order, the pairs in turn.  With skewed groups and more than one round of tiles:
+// largest groups first, the pairs back and forth.  A tile of 512 rows takes four times one of 128, and in the groups' own
+// order one pair got two of the largest while others had none (gate/up, us, own order | by size, on the single-CTA kernel:
+// 16 groups, 1024 Zipf-distributed rows, K 768, N 768: 23.4 | 19.7, 17.5; 32 groups, 10296 rows, K 1280, N 640: 59.3 | 46.4,
+// 47.0; 128 groups, 131072 rows, K 2048, N 768: 661 | 639, 678).
 struct PairTable {
   const int* off;                                // [E + 1]
-  const int* first;                              // [E + 1]: first tile of the group
+  const int* group;                              // [E]: the groups by size, or null: in their own order
+  const int* first;                              // [E + 1]: first tile of the group in that order
   int E, units;
   __device__ static int shape_of(int n) { return n <= 128 ? DEEP : n <= PN ? WEIGHTS2 : TOKENS2; }
   __device__ static int tiles_of(int n, int units) {
@@ -166,14 +173,14 @@ struct PairTable {
       const int mid = (lo + hi) >> 1;
       if (first[mid] <= t) lo = mid; else hi = mid;
     }
-    const int n = off[lo + 1] - off[lo], local = t - first[lo];
+    const int local = t - first[lo], e = group != nullptr ? group[lo] : lo, n = off[e + 1] - off[e];
     PairTile w;
-    w.expert = lo;
+    w.expert = e;
     w.shape = shape_of(n);
     if (w.shape != TOKENS2) {
       w.unit = w.shape == WEIGHTS2 ? 2 * local : local;
       w.two = w.shape == WEIGHTS2 && w.unit + 1 < units;
-      w.tok0 = off[lo];
+      w.tok0 = off[e];
       w.ntok = n;
       w.n0 = (n + 31) & ~31;
       w.n1 = 0;
@@ -181,7 +188,7 @@ struct PairTable {
       const int ntt = (n + 2 * PN - 1) / (2 * PN), tt = local / units;
       const int width = (((n + ntt - 1) / ntt) + 31) & ~31;      // balanced token tiles, at most 512 rows
       w.unit = local - tt * units;
-      w.tok0 = off[lo] + tt * width;
+      w.tok0 = off[e] + tt * width;
       w.ntok = min(width, n - tt * width);
       w.n0 = (((w.ntok + 1) >> 1) + 31) & ~31;
       w.n1 = w.ntok > w.n0 ? (w.ntok - w.n0 + 31) & ~31 : 0;
@@ -220,6 +227,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * (2 * P_NST + 4) + 8);
   int* s_off = reinterpret_cast<int*>(bar_mem + 256);
   int* s_first = s_off + P.E + 1;
+  int* s_group = s_first + P.E + 1;
+  volatile int* skew_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * (2 * P_NST + 4) + 12);
 
   const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int rank = (int)uniform(cluster_rank());
@@ -245,29 +254,58 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   }
   for (int e = threadIdx.x; e <= E; e += blockDim.x) s_off[e] = P.offsets[e];
   __syncthreads();
-  if (warp == 0) {                               // first[]: exclusive sums of the groups' tile counts
-    int carry = 0;
+  const int pairs = (int)(gridDim.x >> 1), pair = (int)(blockIdx.x >> 1);
+  // first[]: exclusive sums of the groups' tile counts; the largest group's rows
+  auto count_tiles = [&](const int* order) {
+    int carry = 0, most = 0;
     for (int e0 = 0; e0 < E; e0 += 32) {
-      const int e = e0 + lane;
-      const int c = e < E ? PairTable::tiles_of(s_off[e + 1] - s_off[e], units) : 0;
+      const int at = e0 + lane, e = order != nullptr && at < E ? order[at] : at;
+      const int n = at < E ? s_off[e + 1] - s_off[e] : 0, c = PairTable::tiles_of(n, units);
+      most = max(most, n);
       int incl = c;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      if (e < E) s_first[e] = carry + incl - c;
+      if (at < E) s_first[at] = carry + incl - c;
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (lane == 0) s_first[E] = carry;
+    return __reduce_max_sync(0xffffffffu, most);
+  };
+  if (warp == 0) {
+    const int most = count_tiles(nullptr);
+    // skewed: the largest group is over twice the average
+    if (lane == 0) *skew_flag = E <= P_SORT_E && s_first[E] > pairs && most > PN && most / 2 > (s_off[E] - s_off[0]) / E;
   }
   fence_before_sync();
   __syncthreads();
+  const bool skewed = *skew_flag != 0;
+  if (skewed) {                                  // a group's place is the number of larger ones, equals in their order
+    int n[P_SORT_E / 32];
+#pragma unroll
+    for (int j = 0; j < P_SORT_E / 32; ++j) {
+      const int e = 32 * j + lane;
+      n[j] = e < E ? s_off[e + 1] - s_off[e] : -1;
+    }
+    for (int e = warp; e < E; e += (int)(blockDim.x >> 5)) {
+      const int mine = s_off[e + 1] - s_off[e];
+      int before = 0;
+#pragma unroll
+      for (int j = 0; j < P_SORT_E / 32; ++j) before += n[j] > mine || (n[j] == mine && 32 * j + lane < e) ? 1 : 0;
+      before = __reduce_add_sync(0xffffffffu, before);
+      if (lane == 0) s_group[before] = e;
+    }
+    __syncthreads();
+    if (warp == 0) count_tiles(s_group);
+  }
   cluster_sync();                                // barriers, TMEM and table of both CTAs are ready
   fence_after_sync();
   const uint32_t tmem = uniform(*tmem_ptr);
-  const PairTable table{s_off, s_first, E, units};
-  const int total = s_first[E], pairs = (int)(gridDim.x >> 1), pair = (int)(blockIdx.x >> 1);
+  const PairTable table{s_off, skewed ? s_group : nullptr, s_first, E, units};
+  const int total = s_first[E];
+  auto deal = [&](int i) { return i * pairs + (skewed && (i & 1) != 0 ? pairs - 1 - pair : pair); };   // its i-th tile
 
   if (warp == 0) {
     // ------------------------------------------------------------------ operand copies by TMA
@@ -287,8 +325,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     auto load_b = [&](uint32_t dst, uint32_t bar, int k, int row, int boxes) {
       for (int b = 0; b < boxes; ++b) tma_load_pair(dst + b * P_BOX_BYTES, &map_x, bar, k, row + b * P_BOX);
     };
-    for (int t = pair; t < total && ok; t += pairs) {
-      const PairTile w = table.locate(t);
+    for (int nth = 0; deal(nth) < total && ok; ++nth) {
+      const PairTile w = table.locate(deal(nth));
       const int we = (int)uniform(w.expert % P.period), unit = (int)uniform(w.unit), shape = (int)uniform(w.shape);
       const bool two = uniform(w.two) != 0;
       const int h0 = (int)uniform(w.n0 >> 1), h1 = (int)uniform(w.n1 >> 1);     // this CTA's halves of the token chunks
@@ -334,8 +372,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       int stage = 0, cur = 0;                    // cur: accumulator of the next single-accumulator tile
       uint32_t phase = 0, used = 0;              // used: parity of the tiles each accumulator has held, a bit each
       bool ok = true;
-      for (int t = pair; t < total && ok; t += pairs) {
-        PairTile w = table.locate(t);
+      for (int nth = 0; deal(nth) < total && ok; ++nth) {
+        PairTile w = table.locate(deal(nth));
         w.shape = (int)uniform(w.shape);
         w.two = uniform(w.two) != 0;
         const int b0 = w.two ? 0 : cur;
@@ -426,13 +464,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       }
     };
     if (pair < total) fetch(pair);
-    for (int t = pair; t < total && ok; t += pairs) {
+    for (int nth = 0; deal(nth) < total && ok; ++nth) {
       int row[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) row[i] = next[i] / P.top_k;
       const uint32_t at = at_next;
       const int count = (int)uniform(count_next), step = (int)uniform(step_next);
-      if (t + pairs < total) fetch(t + pairs);   // the next tile's positions travel under this tile's copies
+      if (deal(nth + 1) < total) fetch(deal(nth + 1));   // the next tile's positions travel under this tile's copies
       for (int kb = 0; kb < KB; kb += step) {
         ok = mbar_wait_warp(empty(stage), phase ^ 1u, abort_flag, P.d_status);
         if (!ok) break;
@@ -464,8 +502,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     uint32_t used = 0;
     int cur = 0;
     bool ok = true;
-    for (int t = pair; t < total && ok; t += pairs) {
-      const PairTile w = table.locate(t);
+    for (int nth = 0; deal(nth) < total && ok; ++nth) {
+      const PairTile w = table.locate(deal(nth));
       const int b0 = w.two ? 0 : cur;
       for (int c = 0; c < (w.two ? 2 : 1); ++c) {
         const int b = c == 0 ? b0 : 1;
