@@ -271,19 +271,22 @@ int mq_w4a16_grouped_swiglu(const void* x,
 
 /* The three calls above with a status word: on more than a few rows per group they run a kernel whose bounded waits set
  * MQ_DEV_WAIT_EXPIRED in d_status (may be null) when they run out, and then leave part of the result unwritten.  Without
- * a status word nothing reports that. */
+ * a status word nothing reports that.
+ * rows: how many of the S rows the groups are expected to hold (0: all of them).  The choice of the kernel goes by it, where
+ * S is a buffer's capacity or counts the rows of other ranks' experts too; the result does not depend on it beyond the
+ * order of the fp32 sums. */
 int mq_w4a16_grouped_gemm_ex(const void* x, const int32_t* qweight, const void* scales,
                              const int32_t* qzeros, const int32_t* offsets,
-                             int64_t S, int64_t E, int64_t weight_period, int64_t N, int64_t Kd, int64_t group_size,
-                             void* out, int32_t* d_status, void* stream);
+                             int64_t S, int64_t rows, int64_t E, int64_t weight_period, int64_t N, int64_t Kd,
+                             int64_t group_size, void* out, int32_t* d_status, void* stream);
 int mq_w4a16_linear_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros, int64_t M,
                        int64_t N, int64_t Kd, int64_t group_size, void* out, int32_t* d_status, void* stream);
 int mq_w4a16_grouped_swiglu_ex(const void* x,
                                const int32_t* qweight_gate, const void* scales_gate, const int32_t* qzeros_gate,
                                const int32_t* qweight_up, const void* scales_up, const int32_t* qzeros_up,
                                const int32_t* offsets,
-                               int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H, int64_t group_size,
-                               void* h, int32_t* d_status, void* stream);
+                               int64_t S, int64_t rows, int64_t E, int64_t weight_period, int64_t I, int64_t H,
+                               int64_t group_size, void* h, int32_t* d_status, void* stream);
 
 /* mq_w4a16_grouped_swiglu on rows gathered inside the kernel: row p of the expert-sorted order is x[perm[p] / top_k]
  * of the unpermuted x [T,H] (what mq_permute_plan lists; replaces the row gather of

@@ -176,9 +176,10 @@ extern "C" int mq_moe_forward(const mq_moe_layer* h_layer, const void* x, const 
                                            L.group_size, 0, b.h, d_status, stream));
     } else {
       MQ_BLOCK_STEP(mq_w4a16_grouped_swiglu_ex(b.rows, i32(L.gate[0]), L.gate[1], i32(L.gate[2]), i32(L.up[0]), L.up[1],
-                                               i32(L.up[2]), b.offsets, S, E, E, I, H, L.group_size, b.h, d_status, stream));
+                                               i32(L.up[2]), b.offsets, S, 0, E, E, I, H, L.group_size, b.h, d_status,
+                                               stream));
     }
-    MQ_BLOCK_STEP(mq_w4a16_grouped_gemm_ex(b.h, i32(L.down[0]), L.down[1], i32(L.down[2]), b.offsets, S, E, E, H, I,
+    MQ_BLOCK_STEP(mq_w4a16_grouped_gemm_ex(b.h, i32(L.down[0]), L.down[1], i32(L.down[2]), b.offsets, S, 0, E, E, H, I,
                                            L.group_size, b.y, d_status, stream));
   }
   MQ_BLOCK_STEP(mq_unpermute_combine_residual(b.y, L.dtype, b.weights, b.inv, residual, T, K, H, out, stream));

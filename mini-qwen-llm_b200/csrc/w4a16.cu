@@ -389,15 +389,17 @@ int w4a16_stream(const void* x, const float* xs, int x_format, const int32_t* pe
 bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k, const int32_t* qw0, const void* sc0,
                const int32_t* qz0, const int32_t* qw1, const void* sc1, const int32_t* qz1, bool swiglu,
-               const int32_t* offsets, int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, void* out,
-               int32_t* d_status, cudaStream_t st);
+               const int32_t* offsets, int64_t S, int64_t rows, int64_t E, int64_t period, int64_t N, int64_t Kd,
+               void* out, int32_t* d_status, cudaStream_t st);
 
 namespace {
 
 int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* offsets, int64_t S, int64_t E,
               int64_t period, int64_t N, int64_t Kd, int64_t group, void* out, cudaStream_t st,
               const int32_t* perm = nullptr, int64_t top_k = 1, int32_t* d_status = nullptr,
-              const float* xs = nullptr, int x_format = 0, bool shuffle_out = false, bool want_stream = false) {
+              const float* xs = nullptr, int x_format = 0, bool shuffle_out = false, bool want_stream = false,
+              int64_t rows = 0) {
+  if (rows <= 0 || rows > S) rows = S;            // rows that the groups are expected to hold
   if (S < 0 || E <= 0 || N <= 0 || Kd <= 0 || group <= 0) return MQ_ERR_INVALID_ARGUMENT;
   if (period <= 0 || period > E) return MQ_ERR_INVALID_ARGUMENT;
   if (group % 32 != 0 || Kd % group != 0 || N % 8 != 0 || E > 65535) return MQ_ERR_UNSUPPORTED_SHAPE;
@@ -414,10 +416,10 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
   // dozen slots on (below 32 slots both are bound by launch latency), the per-lane cp.async kernel for the single
   // projection (its K is short and it needs no K split).  The prepared-activation entry points ask for the stream
   // kernel explicitly.
-  if (!want_stream && x_format == 0 && S > 8 * E && w4a16_tile_covers(S, E, period, N, Kd, group) && aligned16(p0.qz) &&
+  if (!want_stream && x_format == 0 && rows > 8 * E && w4a16_tile_covers(S, E, period, N, Kd, group) && aligned16(p0.qz) &&
       (!swiglu || aligned16(p1.qz)) && S * (Kd / 8) < ((int64_t)1 << 32))
-    return w4a16_tile(x, S, nullptr, 1, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, offsets, S, E, period, N, Kd,
-                      out, d_status, st);
+    return w4a16_tile(x, S, nullptr, 1, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, offsets, S, rows, E, period, N,
+                      Kd, out, d_status, st);
   const bool stream = want_stream || (swiglu && S >= 32);
   if (stream && w4a16_stream_covers(S, E, period, N, Kd, group))
     return w4a16_stream(x, xs, x_format, perm, top_k, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, shuffle_out,
@@ -441,19 +443,20 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
 }  // namespace mq
 
 extern "C" int mq_w4a16_grouped_gemm_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
-                                        const int32_t* offsets, int64_t S, int64_t E, int64_t weight_period, int64_t N,
-                                        int64_t Kd, int64_t group_size, void* out, int32_t* d_status, void* stream) {
+                                        const int32_t* offsets, int64_t S, int64_t rows, int64_t E,
+                                        int64_t weight_period, int64_t N, int64_t Kd, int64_t group_size, void* out,
+                                        int32_t* d_status, void* stream) {
   mq::W4Proj p{qweight, reinterpret_cast<const __nv_bfloat16*>(scales), qzeros};
   return mq::launch_w4(x, p, p, false, offsets, S, E, weight_period, N, Kd, group_size, out,
-                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status);
+                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status, nullptr, 0, false, false, rows);
 }
 
 extern "C" int mq_w4a16_grouped_gemm(const void* x, const int32_t* qweight, const void* scales,
                                      const int32_t* qzeros, const int32_t* offsets,
                                      int64_t S, int64_t E, int64_t weight_period, int64_t N, int64_t Kd,
                                      int64_t group_size, void* out, void* stream) {
-  return mq_w4a16_grouped_gemm_ex(x, qweight, scales, qzeros, offsets, S, E, weight_period, N, Kd, group_size, out, nullptr,
-                                  stream);
+  return mq_w4a16_grouped_gemm_ex(x, qweight, scales, qzeros, offsets, S, 0, E, weight_period, N, Kd, group_size, out,
+                                  nullptr, stream);
 }
 
 extern "C" int mq_w4a16_linear_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
@@ -473,12 +476,12 @@ extern "C" int mq_w4a16_grouped_swiglu_ex(const void* x,
                                           const int32_t* qweight_gate, const void* scales_gate,
                                           const int32_t* qzeros_gate, const int32_t* qweight_up, const void* scales_up,
                                           const int32_t* qzeros_up, const int32_t* offsets,
-                                          int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H,
-                                          int64_t group_size, void* h, int32_t* d_status, void* stream) {
+                                          int64_t S, int64_t rows, int64_t E, int64_t weight_period, int64_t I,
+                                          int64_t H, int64_t group_size, void* h, int32_t* d_status, void* stream) {
   mq::W4Proj p0{qweight_gate, reinterpret_cast<const __nv_bfloat16*>(scales_gate), qzeros_gate};
   mq::W4Proj p1{qweight_up, reinterpret_cast<const __nv_bfloat16*>(scales_up), qzeros_up};
   return mq::launch_w4(x, p0, p1, true, offsets, S, E, weight_period, I, H, group_size, h,
-                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status);
+                       reinterpret_cast<cudaStream_t>(stream), nullptr, 1, d_status, nullptr, 0, false, false, rows);
 }
 
 extern "C" int mq_w4a16_grouped_swiglu(const void* x,
@@ -488,7 +491,7 @@ extern "C" int mq_w4a16_grouped_swiglu(const void* x,
                                        int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H,
                                        int64_t group_size, void* h, void* stream) {
   return mq_w4a16_grouped_swiglu_ex(x, qweight_gate, scales_gate, qzeros_gate, qweight_up, scales_up, qzeros_up, offsets, S,
-                                    E, weight_period, I, H, group_size, h, nullptr, stream);
+                                    0, E, weight_period, I, H, group_size, h, nullptr, stream);
 }
 
 extern "C" int mq_w4a16_grouped_swiglu_gather(const void* x, const int32_t* perm,
@@ -508,7 +511,7 @@ extern "C" int mq_w4a16_grouped_swiglu_gather(const void* x, const int32_t* perm
     if (p == nullptr || !aligned16(p)) return MQ_ERR_INVALID_ARGUMENT;
   if (!perm || !offsets) return MQ_ERR_INVALID_ARGUMENT;
   return w4a16_tile(x, T, perm, top_k, qweight_gate, scales_gate, qzeros_gate, qweight_up, scales_up, qzeros_up, true,
-                    offsets, S, E, weight_period, I, H, h, d_status, reinterpret_cast<cudaStream_t>(stream));
+                    offsets, S, S, E, weight_period, I, H, h, d_status, reinterpret_cast<cudaStream_t>(stream));
 }
 
 /* Prepared-activation forms: see include/mqmoe.h. */

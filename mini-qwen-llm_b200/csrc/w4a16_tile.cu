@@ -518,11 +518,12 @@ bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t 
 
 bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 
-// x: rows in natural k order, [S, Kd] or (perm) [x_rows, Kd] gathered by row = perm[p] / top_k.
+// x: rows in natural k order, [S, Kd] or (perm) [x_rows, Kd] gathered by row = perm[p] / top_k.  `rows` of the S rows are
+// expected to lie in the groups.
 int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k, const int32_t* qw0, const void* sc0,
                const int32_t* qz0, const int32_t* qw1, const void* sc1, const int32_t* qz1, bool swiglu,
-               const int32_t* offsets, int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, void* out,
-               int32_t* d_status, cudaStream_t st) {
+               const int32_t* offsets, int64_t S, int64_t rows, int64_t E, int64_t period, int64_t N, int64_t Kd,
+               void* out, int32_t* d_status, cudaStream_t st) {
   if (x_rows * (Kd / 8) >= ((int64_t)1 << 32)) return MQ_ERR_UNSUPPORTED_SHAPE;
   if ((reinterpret_cast<uintptr_t>(qz0) & 15u) != 0 || (swiglu && (reinterpret_cast<uintptr_t>(qz1) & 15u) != 0))
     return MQ_ERR_INVALID_ARGUMENT;
@@ -546,8 +547,9 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
   P.out = reinterpret_cast<__nv_bfloat16*>(out);
   P.d_status = d_status;
   const int sms = device_sm_count();
-  // Most token tiles there can be, with tiles of tn tokens.
-  auto token_tiles = [&](int64_t tn) { return (S + tn - 1) / tn + (E > 1 ? (E < S ? E : S) : 0); };
+  // Most token tiles there can be in n rows, with tiles of tn tokens.
+  auto most_tiles = [&](int64_t n, int64_t tn) { return (n + tn - 1) / tn + (E > 1 ? (E < n ? E : n) : 0); };
+  auto token_tiles = [&](int64_t tn) { return most_tiles(rows, tn); };
   // Plain projection: 256 columns per tile as long as that leaves a tile for every SM; otherwise 128, and narrower
   // token tiles while there is less than a tile per SM (a tile's time hardly depends on its tokens below 64).
   const bool wide = !swiglu && token_tiles(TL_TN) * ((N + 255) / 256) >= sms;
@@ -555,7 +557,7 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
   int tn = TL_TN;
   while (tn > 32 && token_tiles(tn) * col_tiles < sms && token_tiles(tn / 2) * col_tiles <= sms) tn /= 2;
   P.tn = tn;
-  const int64_t tiles = token_tiles(tn) * col_tiles;
+  const int64_t tiles = most_tiles(S, tn) * col_tiles;
   const int grid = (int)(tiles < sms ? tiles : sms);
 #define MQ_TILE_LAUNCH(MODE, GATHER)                                                                                \
   do {                                                                                                              \

@@ -43,9 +43,9 @@ PROTOTYPES = {
     "mq_w4a16_grouped_gemm": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_linear": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_grouped_swiglu": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
-    "mq_w4a16_grouped_gemm_ex": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
+    "mq_w4a16_grouped_gemm_ex": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_linear_ex": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _P, _P, _P]),
-    "mq_w4a16_grouped_swiglu_ex": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
+    "mq_w4a16_grouped_swiglu_ex": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_grouped_swiglu_gather": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_stream_swiglu": (c_int, [_P, _P, _I, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _I, _P, _P, _P]),
     "mq_w4a16_stream_gemm": (c_int, [_P, _P, _I, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P, _P]),

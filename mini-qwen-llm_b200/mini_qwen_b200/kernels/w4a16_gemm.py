@@ -42,10 +42,11 @@ def _check_w4(x, qweight, scales, qzeros, group_size, E, prepared_f16=False):
 
 def w4a16_grouped_gemm(x, qweight, scales, qzeros, expert_offsets, group_size: int = 128,
                        zero_init: bool = True, out: torch.Tensor | None = None,
-                       status: torch.Tensor | None = None) -> torch.Tensor:
+                       status: torch.Tensor | None = None, rows: int = 0) -> torch.Tensor:
     """Rows ``offsets[e]:offsets[e+1]`` of x times the dequantised weight of expert e.
     qweight [E, K/8, N], scales [E, K/g, N], qzeros [E, K/g, N/8], offsets int32 [E+1].  ``status`` (int32 [1],
-    optional) receives device-side error bits (a bounded wait that ran out)."""
+    optional) receives device-side error bits (a bounded wait that ran out).  ``rows``: how many of x's rows the groups are
+    expected to hold, where x is a buffer or holds other ranks' rows too (0: all); the choice of the kernel goes by it."""
     E = qweight.shape[0]
     K, N = _check_w4(x, qweight, scales, qzeros, group_size, E)
     expert_offsets = _offsets32(expert_offsets)
@@ -57,16 +58,16 @@ def w4a16_grouped_gemm(x, qweight, scales, qzeros, expert_offsets, group_size: i
         out = (torch.zeros if zero_init else torch.empty)(S, N, dtype=torch.bfloat16, device=x.device)
     assert out.is_contiguous() and tuple(out.shape) == (S, N) and out.dtype == torch.bfloat16
     rc = _cabi.load().mq_w4a16_grouped_gemm_ex(_cabi.ptr(x), _cabi.ptr(qweight), _cabi.ptr(scales), _cabi.ptr(qzeros),
-                                               _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(out),
-                                               _cabi.ptr(status), _cabi.stream_ptr(x.device))
+                                               _cabi.ptr(expert_offsets), S, rows, groups, E, N, K, group_size,
+                                               _cabi.ptr(out), _cabi.ptr(status), _cabi.stream_ptr(x.device))
     _cabi.check(rc, "mq_w4a16_grouped_gemm")
     _cabi.count_launches(1 if S else 0)
     return out
 
 
 def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zero_init: bool = True,
-                         status: torch.Tensor | None = None) -> torch.Tensor:
-    """Fused gate/up W4A16 projections + SwiGLU; gate and up are (qweight, scales, qzeros) stacks; ``status`` as in
+                         status: torch.Tensor | None = None, rows: int = 0) -> torch.Tensor:
+    """Fused gate/up W4A16 projections + SwiGLU; gate and up are (qweight, scales, qzeros) stacks; ``status`` and ``rows`` as in
     :func:`w4a16_grouped_gemm`."""
     E = gate[0].shape[0]
     K, N = _check_w4(x, *gate, group_size, E)
@@ -79,7 +80,7 @@ def w4a16_grouped_swiglu(x, gate, up, expert_offsets, group_size: int = 128, zer
     h = (torch.zeros if zero_init else torch.empty)(S, N, dtype=torch.bfloat16, device=x.device)
     rc = _cabi.load().mq_w4a16_grouped_swiglu_ex(
         _cabi.ptr(x), _cabi.ptr(gate[0]), _cabi.ptr(gate[1]), _cabi.ptr(gate[2]), _cabi.ptr(up[0]), _cabi.ptr(up[1]),
-        _cabi.ptr(up[2]), _cabi.ptr(expert_offsets), S, groups, E, N, K, group_size, _cabi.ptr(h), _cabi.ptr(status),
+        _cabi.ptr(up[2]), _cabi.ptr(expert_offsets), S, rows, groups, E, N, K, group_size, _cabi.ptr(h), _cabi.ptr(status),
         _cabi.stream_ptr(x.device))
     _cabi.check(rc, "mq_w4a16_grouped_swiglu")
     _cabi.count_launches(1 if S else 0)

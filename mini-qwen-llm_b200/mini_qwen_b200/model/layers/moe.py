@@ -461,16 +461,17 @@ class Qwen3MoEBlock(nn.Module):
                     return out
         return self.forward(norm(h), residual=h)
 
-    def _experts(self, st, rows, off32, out=None):
-        """Grouped gate/up + SwiGLU and down projection over rows grouped by `off32`."""
+    def _experts(self, st, rows, off32, out=None, expected: int = 0):
+        """Grouped gate/up + SwiGLU and down projection over rows grouped by `off32`, which are expected to be `expected`
+        of the rows there are (0: all)."""
         run = self._stage
         # the groups of a routing cover every row that is read later, so no output needs a zero fill
         status = self._status_word(rows.device)
         if st["w4"]:
             h = run("grouped_swiglu", w4a16_grouped_swiglu, rows, st["gate_proj"], st["up_proj"], off32,
-                    st["group_size"], zero_init=False, status=status)
+                    st["group_size"], zero_init=False, status=status, rows=expected)
             return run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off32, st["group_size"],
-                       zero_init=False, out=out, status=status)
+                       zero_init=False, out=out, status=status, rows=expected)
         h = run("grouped_swiglu", moe_grouped_swiglu, rows, st["w13"], off32, zero_init=False, status=status)
         return run("grouped_down", moe_grouped_gemm, h, st["w2"], off32, zero_init=False, out=out, status=status)
 
@@ -567,8 +568,9 @@ class Qwen3MoEBlock(nn.Module):
         status = self._status_word(x2d.device)
         h = run("grouped_swiglu", w4a16_stream_swiglu, xp_tok, xs_tok, st["gate_proj"], st["up_proj"], off_local,
                 st["group_size"], shuffle_out=False, status=status, perm=perm, top_k=K)
+        # of the G*T tokens' slots a rank's experts own one in G on average
         out_perm = run("grouped_down", w4a16_grouped_gemm, h, *st["down_proj"], off_local, st["group_size"],
-                       zero_init=False, status=status)
+                       zero_init=False, status=status, rows=max(1, T * K))
         run("send_partials", peer.send_partials, out_perm, weights, ids32, inv, T, K, el)   # barrier inside
         return run("sum_partials", peer.sum_partials, T, res)
 
@@ -608,7 +610,8 @@ class Qwen3MoEBlock(nn.Module):
             run("grouped_down", moe_grouped_gemm, h, st["w2"], seg, zero_init=False, out=peer.y_rows(), status=status)
             run("rank_barrier", peer.rank_barrier)
             return run("combine", peer.combine, weights, inv, slot_dst, T, K, residual=res)
-        self._experts(st, peer.recv_rows(), seg, out=peer.y_rows())
+        # the receive buffer has room for every rank's slots; on average a rank gets as many as it sends
+        self._experts(st, peer.recv_rows(), seg, out=peer.y_rows(), expected=T * K)
         run("rank_barrier", peer.rank_barrier)
         return run("combine", peer.combine, weights, inv, slot_dst, T, K, residual=res)
 

@@ -327,3 +327,38 @@ def test_zero_points_off_the_16_byte_grid_keep_a_layer_off_the_tile_kernel():
         assert blk._w4_tile(st, 1000) is want
         st["gate_proj"], st["up_proj"] = (st["gate_proj"][0], None, flat[at:]), (None, None, flat[off:])
         assert blk._w4_tile(st, 1000) is want
+
+
+def test_expert_parallel_w4a16_calls_say_how_many_rows_are_a_ranks_own(monkeypatch):
+    """Decode by replication hands over all ranks' slots, the peer path a buffer with room for them; the choice of the
+    kernels goes by the slots that one rank's experts own on average."""
+    from mini_qwen_b200.model.layers import moe
+    T, K, E, G, H, I = 8, 2, 16, 4, 64, 32
+    blk = Qwen3MoEBlock(Qwen3MoEConfig(hidden_size=H, intermediate_size=I, num_experts=E, num_experts_per_tok=K))
+    blk.ep_size, blk.ep_rank, blk.num_local_experts = G, 1, E // G
+    st = {"w4": True, "group_size": 32, "gate_proj": (), "up_proj": (), "down_proj": (torch.zeros(1),) * 3}
+    seen = []
+
+    class Peer:
+        def gather_tokens(self, x):
+            return x.repeat(G, 1)
+
+        def recv_rows(self):
+            return torch.zeros(G * T * K, H, dtype=torch.bfloat16)
+
+        def __getattr__(self, name):
+            return (lambda *a, **k: (None, None)) if name == "exchange_plan" else (lambda *a, **k: torch.zeros(1))
+    blk._ensure_peer = lambda *a: Peer()
+    blk._status_word = lambda device: torch.zeros(1, dtype=torch.int32)
+    off = torch.arange(E + 1, dtype=torch.int32)
+    monkeypatch.setattr(moe, "route_small_workspace", lambda *a: torch.zeros(1))
+    monkeypatch.setattr(moe, "moe_route_small", lambda x, *a, **k: (None, None, None, None, off, x, x))
+    monkeypatch.setattr(moe, "w4a16_stream_swiglu", lambda xp, *a, **k: xp)
+    monkeypatch.setattr(moe, "w4a16_grouped_swiglu", lambda x, *a, **k: seen.append((x.shape[0], k["rows"])) or x)
+    monkeypatch.setattr(moe, "w4a16_grouped_gemm", lambda x, *a, **k: seen.append((x.shape[0], k["rows"])) or x)
+    x = torch.zeros(T, H, dtype=torch.bfloat16)
+    blk._forward_replicated(x, st, T, K, E)
+    assert seen == [(G * T, T * K)]
+    seen.clear()
+    blk._forward_peer(x, st, None, None, None, None, off, T, K, E)
+    assert seen == [(G * T * K, T * K)] * 2
