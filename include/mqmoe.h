@@ -269,6 +269,11 @@ int mq_w4a16_grouped_swiglu(const void* x,
                             int64_t S, int64_t E, int64_t weight_period, int64_t I, int64_t H, int64_t group_size,
                             void* h, void* stream);
 
+/* Whether `rows` rows in `groups` groups go to the tensor-core tile kernel (1) or to the kernels that stream the weights
+ * for every eight rows (0): what the calls here decide by, from sizes alone.  swiglu: the fused gate/up projection;
+ * prepare: its alternative would need the activations prepared by a launch of its own. */
+int mq_w4a16_tile_pays(int64_t rows, int64_t groups, int64_t N, int64_t Kd, int64_t group_size, int swiglu, int prepare);
+
 /* The three calls above with a status word: on more than a few rows per group they run a kernel whose bounded waits set
  * MQ_DEV_WAIT_EXPIRED in d_status (may be null) when they run out, and then leave part of the result unwritten.  Without
  * a status word nothing reports that.

@@ -17,7 +17,6 @@ int grouped_gemm_generic_dispatch(const void* a, const void* w, const int32_t* o
                                   int64_t period, int64_t N, int64_t Kd, int dtype, bool swiglu, void* out,
                                   cudaStream_t st, const int32_t* perm, int64_t top_k);
 bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
-bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 
 namespace {
 
@@ -33,12 +32,14 @@ BlockPlan plan_of(const mq_moe_layer& L, int64_t T) {
   // decode batches: logits, top-k, plan (and the W4A16 activation preparation) in one launch
   p.small = T <= 64 && E <= 256 && K <= 32 && S <= 2048;
   if (p.w4) {
-    // more than eight rows per expert on average: the tile kernel (the rule of the W4A16 dispatch), whose bulk copies
-    // want the zero points 16-byte aligned; the other kernels read them word by word
-    p.tile = S > 8 * E && w4a16_tile_covers(S, E, E, I, H, L.group_size) && T * (H / 8) < ((int64_t)1 << 32) &&
+    const bool streams = H <= 4096 && w4a16_stream_covers(S, E, E, I, H, L.group_size);
+    const bool prepared = streams && p.small && T <= E;         // by the routing launch
+    // The tile kernel by the rule of the W4A16 dispatch.  Its bulk copies want the zero points 16-byte aligned; the other
+    // kernels read them word by word.
+    p.tile = mq_w4a16_tile_pays(S, E, I, H, L.group_size, 1, !prepared) && T * (H / 8) < ((int64_t)1 << 32) &&
              aligned16(L.gate[2]) && aligned16(L.up[2]);
-    p.stream = !p.tile && H <= 4096 && w4a16_stream_covers(S, E, E, I, H, L.group_size);
-    p.prepared = p.stream && p.small && T <= E;
+    p.stream = !p.tile && streams;
+    p.prepared = !p.tile && prepared;
     p.gather_in_kernel = p.tile || p.stream;
   } else {
     p.tc5 = L.dtype == MQ_BF16 && tc5_covers(S, E, I, H, true) && T * H < ((int64_t)1 << 32);

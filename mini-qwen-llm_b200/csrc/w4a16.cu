@@ -387,6 +387,7 @@ int w4a16_stream(const void* x, const float* xs, int x_format, const int32_t* pe
 
 // Tensor-core tile kernel for prefill-size groups (w4a16_tile.cu).
 bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
+bool w4a16_tile_faster(int64_t rows, int64_t E, int64_t N, int64_t Kd, bool swiglu, int alternative);
 int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k, const int32_t* qw0, const void* sc0,
                const int32_t* qz0, const int32_t* qw1, const void* sc1, const int32_t* qz1, bool swiglu,
                const int32_t* offsets, int64_t S, int64_t rows, int64_t E, int64_t period, int64_t N, int64_t Kd,
@@ -409,14 +410,14 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
   if (swiglu && (!p1.qw || !p1.sc || !p1.qz)) return MQ_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(p0.qw) || !aligned16(p0.sc) || !aligned16(out)) return MQ_ERR_INVALID_ARGUMENT;
   if (swiglu && (!aligned16(p1.qw) || !aligned16(p1.sc))) return MQ_ERR_INVALID_ARGUMENT;
-  // Which kernel.  More than one block of eight rows per group on average: the tensor-core tile kernel, which
-  // unpacks a weight once for up to 128 rows (gate/up of the 128-expert layer, cold: 94 against 106 us at 128 tokens,
-  // 125 against 107 at 192; a 2048 x 4096 linear: 12.4 against 17.4 us at 8 rows, 17.4 against 17.4 at 9, 115 against
-  // 18 at 64).  Below that the TMA-staged stream kernel is the faster one for the fused gate/up projection from a few
-  // dozen slots on (below 32 slots both are bound by launch latency), the per-lane cp.async kernel for the single
-  // projection (its K is short and it needs no K split).  The prepared-activation entry points ask for the stream
-  // kernel explicitly.
-  if (!want_stream && x_format == 0 && rows > 8 * E && w4a16_tile_covers(S, E, period, N, Kd, group) && aligned16(p0.qz) &&
+  // Which kernel.  The tensor-core tile kernel where it is the faster one (from about nine rows a group on, see its rule;
+  // more groups than the stream kernel takes: from eight on).  Otherwise the TMA-staged stream kernel for the fused
+  // gate/up projection from a few dozen slots on (below 32 slots both are bound by launch latency), the per-lane cp.async
+  // kernel for the single projection (its K is short and it needs no K split).  The prepared-activation entry points ask
+  // for the stream kernel explicitly.
+  const bool faster = swiglu && !w4a16_stream_covers(S, E, period, N, Kd, group)
+                          ? rows > 8 * E : w4a16_tile_faster(rows, E, N, Kd, swiglu, 0);
+  if (!want_stream && x_format == 0 && faster && w4a16_tile_covers(S, E, period, N, Kd, group) && aligned16(p0.qz) &&
       (!swiglu || aligned16(p1.qz)) && S * (Kd / 8) < ((int64_t)1 << 32))
     return w4a16_tile(x, S, nullptr, 1, p0.qw, p0.sc, p0.qz, p1.qw, p1.sc, p1.qz, swiglu, offsets, S, rows, E, period, N,
                       Kd, out, d_status, st);
@@ -441,6 +442,16 @@ int launch_w4(const void* x, W4Proj p0, W4Proj p1, bool swiglu, const int32_t* o
 
 }  // namespace
 }  // namespace mq
+
+extern "C" int mq_w4a16_tile_pays(int64_t rows, int64_t groups, int64_t N, int64_t Kd, int64_t group_size, int swiglu,
+                                  int prepare) {
+  using namespace mq;
+  if (rows <= 0 || groups <= 0 || N <= 0 || Kd <= 0 || group_size <= 0 ||
+      !w4a16_tile_covers(rows, groups, groups, N, Kd, group_size))
+    return 0;
+  if (swiglu && !w4a16_stream_covers(rows, groups, groups, N, Kd, group_size)) return rows > 8 * groups;
+  return w4a16_tile_faster(rows, groups, N, Kd, swiglu != 0, prepare != 0 ? 2 : 1);
+}
 
 extern "C" int mq_w4a16_grouped_gemm_ex(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
                                         const int32_t* offsets, int64_t S, int64_t rows, int64_t E,

@@ -726,6 +726,19 @@ bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_
   return true;
 }
 
+// Column panels of an item: as many as still leave about four items per SM.  The number of experts hit is at most
+// min(E, S), and every one of them has at least one block of rows.
+int w4a16_stream_panels(int64_t S, int64_t E, int64_t N, bool swiglu) {
+  const int64_t active = S < E ? S : E, panels = N / 32;
+  for (int c : {16, 8, 4, 2}) {
+    if (swiglu && c >= 8) continue;                 // a gate + up stage of 8 panels would not fit the ring
+    const int64_t items = active * ((panels + c - 1) / c);
+    // 16 panels = no K split at all (no partial sums to add up): worth fewer items per SM
+    if (items >= (c == 16 ? 3 : 4) * ws_sm_count()) return c;
+  }
+  return 1;
+}
+
 // x: activations; perm != nullptr gathers row p of the sorted order from x[perm[p] / top_k].
 // x_format: 0 = bf16 rows in natural k order; 1 = bf16 rows with the k order 0,4,1,5,2,6,3,7 inside every 8;
 // 2 = that order in fp16, every row scaled by its power of two (needs xs); xs (optional): group sums of the rows
@@ -739,17 +752,8 @@ int w4a16_stream(const void* x, const float* xs, int x_format, const int32_t* pe
   const int G = (int)(Kd / 128);
   const int nproj = swiglu ? 2 : 1;
   if (xs != nullptr && G > 32) return MQ_ERR_UNSUPPORTED_SHAPE;       // the sums table has 32 groups per row
-  // Column panels per item: as many as still leave about four items per SM.  The number of experts hit is
-  // at most min(E, S), and every one of them has at least one block of rows.
-  const int64_t active = S < E ? S : E;
   const int64_t panels = N / 32;
-  int CW = 1;
-  for (int c : {16, 8, 4, 2}) {
-    if (swiglu && c >= 8) continue;                 // a gate + up stage of 8 panels would not fit the ring
-    const int64_t items = active * ((panels + c - 1) / c);
-    // 16 panels = no K split at all (no partial sums to add up): worth fewer items per SM
-    if (items >= (c == 16 ? 3 : 4) * ws_sm_count()) { CW = c; break; }
-  }
+  const int CW = w4a16_stream_panels(S, E, N, swiglu);
   const int KW = WS_CONSUMERS / CW;
   // groups per warp and stage: as many as keep a stage within 64 KB (SwiGLU: two projections) / 96 KB
   const int per_group_bytes = nproj * 128 * 16 * KW * CW;          // stage bytes for gpw = 1

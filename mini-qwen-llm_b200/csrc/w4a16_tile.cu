@@ -21,6 +21,8 @@
 // Modes: SWIGLU folds gate and up of the same 128 columns; WIDE two neighbouring 128-column tiles (a token tile is
 // then fetched once for 256 columns); NARROW one tile (more CTAs where columns x tokens leave SMs idle).
 // Register shares of the five warpgroups: 3 x 40 + 2 x 176 (the masters), within the launch's 5 x 96.
+#include <cmath>
+
 #include "tc5.cuh"
 
 namespace mq {
@@ -511,12 +513,73 @@ bool tile_map_x(CUtensorMap* map, const void* x, int64_t rows, int64_t Kd) {
 
 }  // namespace
 
+bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
+int w4a16_stream_panels(int64_t S, int64_t E, int64_t N, bool swiglu);
+
+namespace {
+
+// How a call is cut into tiles.  Plain projection: 256 columns per tile as long as that leaves a tile for every SM;
+// otherwise 128, and narrower token tiles while there is less than a tile per SM (a tile's time hardly depends on its
+// tokens below 64).
+struct TileShape {
+  bool wide;
+  int tn;                                        // most tokens per tile
+  int64_t col_tiles;
+};
+// Most token tiles there can be in S rows, with tiles of tn tokens.
+int64_t most_token_tiles(int64_t S, int64_t E, int64_t tn) { return (S + tn - 1) / tn + (E > 1 ? (E < S ? E : S) : 0); }
+TileShape tile_shape(int64_t rows, int64_t E, int64_t N, bool swiglu, int sms) {
+  auto token_tiles = [&](int64_t tn) { return most_token_tiles(rows, E, tn); };
+  TileShape t;
+  t.wide = !swiglu && token_tiles(TL_TN) * ((N + 255) / 256) >= sms;
+  t.col_tiles = t.wide ? (N + 255) / 256 : (N + 127) / 128;
+  t.tn = TL_TN;
+  while (t.tn > 32 && token_tiles(t.tn) * t.col_tiles < sms && token_tiles(t.tn / 2) * t.col_tiles <= sms) t.tn /= 2;
+  return t;
+}
+
+}  // namespace
+
+// Whether this kernel is the faster one for `rows` rows in E groups (by the sizes alone; w4a16_tile_covers says whether
+// it takes them).  It unpacks a weight once for up to 128 rows where the others do for every eight, but its units of 128
+// columns x 128 k run one after the other: a tile takes half a microsecond a unit however few its rows.  So the two are
+// compared by their times in us.  The figures are fits to 960 calls of 1 to 128 groups of over 8 to 100 rows (K and N 128
+// to 4096, even and skewed).  Fused, as a block calls it: the slower kernel is chosen by more than 4 % for 6 of 261, by
+// 15 % at most; by the eight rows alone for 32, up to 1.75 times as long (16 groups of 14 rows, K 2048, N 128: 12.2 us on
+// the stream kernel, 21.4 on this; one group of 32 rows, N 768: 7.5 | 20.1).  Plain: for 23 of 697, most of them of K 128,
+// where skewed groups, which a rule on sizes does not see, make the cp.async kernel up to 3.6 times slower.
+// alternative: the fused projection's other kernel: 0 stream or (under 32 rows) cp.async, as the dispatch has it; 1 stream
+// on activations that are prepared already; 2 stream after a launch that prepares them.
+bool w4a16_tile_faster(int64_t rows, int64_t E, int64_t N, int64_t Kd, bool swiglu, int alternative) {
+  if (rows <= 8 * E) return false;               // one block of eight rows a group: a weight is unpacked once anyway
+  const int sms = device_sm_count();
+  const TileShape t = tile_shape(rows, E, N, swiglu, sms);
+  const double units = (double)(Kd / TL_K) * (swiglu || t.wide ? 2 : 1), k = (double)Kd;
+  const int64_t group_tiles = E * ((rows + TL_TN * E - 1) / (TL_TN * E)) * t.col_tiles;      // groups of equal size
+  const double rounds = (double)((group_tiles + sms - 1) / sms), per_group = (double)rows / (8.0 * E);
+  const double blocks = ceil(E == 1 ? per_group : per_group + 0.55);       // of eight rows, in the larger groups
+  if (swiglu) {
+    const double tile = 3.0 + rounds * (0.55 * units + 2.0);
+    if (rows < 32 && alternative == 0) return tile < 2.3 + blocks * (1.7 + 0.0019 * k);
+    // the stream kernel: items of eight rows x `panels` of 32 columns, dealt out to all SMs
+    const int panels = w4a16_stream_panels(rows, E, N, true);
+    const double items = (E == 1 ? ceil(per_group) : (per_group + 0.6) * E) * (double)((N / 32 + panels - 1) / panels);
+    double waves = items / sms;
+    waves = waves < 3.0 ? ceil(waves) : waves + 0.5;
+    return tile < 3.0 + (alternative == 2 ? 2.0 : 0.0) + waves * (2.0 + 0.0013 * k * panels);
+  }
+  const double tile = 2.7 + rounds * (0.5 * units + 2.0), words = (double)N * k * E;
+  if (rows <= 32)                                // the cp.async kernel with K split over four warps
+    return tile < 2.3 + blocks * (1.1 + 0.0017 * k) + words / 7e6;
+  // and without: a warp takes a group's blocks of eight rows one after the other
+  const double even = 5.7 + 0.0025 * k + (per_group + 0.4) * words / 4.5e6, chain = 4.0 + (per_group + 0.5) * 0.006 * k;
+  return tile < (even > chain ? even : chain);
+}
+
 bool w4a16_tile_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group) {
   return group == 128 && Kd % 128 == 0 && N % 32 == 0 && E <= TL_MAX_E && S < ((int64_t)1 << 30) &&
          period * (Kd / 8) < ((int64_t)1 << 31) && (S / 16 + E) * (N / 32) < ((int64_t)1 << 30);
 }
-
-bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group);
 
 // x: rows in natural k order, [S, Kd] or (perm) [x_rows, Kd] gathered by row = perm[p] / top_k.  `rows` of the S rows are
 // expected to lie in the groups.
@@ -547,17 +610,9 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
   P.out = reinterpret_cast<__nv_bfloat16*>(out);
   P.d_status = d_status;
   const int sms = device_sm_count();
-  // Most token tiles there can be in n rows, with tiles of tn tokens.
-  auto most_tiles = [&](int64_t n, int64_t tn) { return (n + tn - 1) / tn + (E > 1 ? (E < n ? E : n) : 0); };
-  auto token_tiles = [&](int64_t tn) { return most_tiles(rows, tn); };
-  // Plain projection: 256 columns per tile as long as that leaves a tile for every SM; otherwise 128, and narrower
-  // token tiles while there is less than a tile per SM (a tile's time hardly depends on its tokens below 64).
-  const bool wide = !swiglu && token_tiles(TL_TN) * ((N + 255) / 256) >= sms;
-  const int64_t col_tiles = wide ? (N + 255) / 256 : (N + 127) / 128;
-  int tn = TL_TN;
-  while (tn > 32 && token_tiles(tn) * col_tiles < sms && token_tiles(tn / 2) * col_tiles <= sms) tn /= 2;
-  P.tn = tn;
-  const int64_t tiles = most_tiles(S, tn) * col_tiles;
+  const TileShape shape = tile_shape(rows, E, N, swiglu, sms);
+  P.tn = shape.tn;
+  const int64_t tiles = most_token_tiles(S, E, shape.tn) * shape.col_tiles;
   const int grid = (int)(tiles < sms ? tiles : sms);
 #define MQ_TILE_LAUNCH(MODE, GATHER)                                                                                \
   do {                                                                                                              \
@@ -571,7 +626,7 @@ int w4a16_tile(const void* x, int64_t x_rows, const int32_t* perm, int64_t top_k
   else if (exact) MQ_TILE_LAUNCH(TILE_SWIGLU_EXACT, false);
   else if (swiglu && perm != nullptr) MQ_TILE_LAUNCH(TILE_SWIGLU, true);
   else if (swiglu) MQ_TILE_LAUNCH(TILE_SWIGLU, false);
-  else if (wide) MQ_TILE_LAUNCH(TILE_WIDE, false);
+  else if (shape.wide) MQ_TILE_LAUNCH(TILE_WIDE, false);
   else MQ_TILE_LAUNCH(TILE_NARROW, false);
 #undef MQ_TILE_LAUNCH
   return check_launch();

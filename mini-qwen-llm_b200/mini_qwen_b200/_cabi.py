@@ -43,6 +43,7 @@ PROTOTYPES = {
     "mq_w4a16_grouped_gemm": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_linear": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _P, _P]),
     "mq_w4a16_grouped_swiglu": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _P, _P]),
+    "mq_w4a16_tile_pays": (c_int, [_L, _L, _L, _L, _L, _I, _I]),
     "mq_w4a16_grouped_gemm_ex": (c_int, [_P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_linear_ex": (c_int, [_P, _P, _P, _P, _L, _L, _L, _L, _P, _P, _P]),
     "mq_w4a16_grouped_swiglu_ex": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _L, _L, _L, _L, _L, _P, _P, _P]),

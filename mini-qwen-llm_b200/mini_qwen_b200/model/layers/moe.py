@@ -24,7 +24,7 @@ from ...kernels.moe_permute import gather_rows, moe_permute_plan
 from ...kernels.moe_router import moe_route_small, moe_router, route_small_supported, route_small_workspace
 from ...kernels.moe_unpermute import unpermute_combine
 from .rms_norm import RMSNorm
-from ...kernels.w4a16_gemm import (w4a16_gather_supported, w4a16_grouped_gemm, w4a16_grouped_swiglu,
+from ...kernels.w4a16_gemm import (w4a16_grouped_gemm, w4a16_grouped_swiglu,
                                      w4a16_grouped_swiglu_gather, w4a16_stream_supported,
                                      w4a16_stream_swiglu, w4a16_tc_gemm, w4a16_tc_prep, w4a16_tc_supported,
                                      w4a16_tc_swiglu)
@@ -403,8 +403,8 @@ class Qwen3MoEBlock(nn.Module):
             h = run("grouped_swiglu", moe_grouped_swiglu_gather, x2d, perm, K, st["w13"], off32, status=status)
             out_perm = run("grouped_down", moe_grouped_gemm, h, st["w2"], off32, zero_init=False, status=status)
             return run("unpermute_combine", unpermute_combine, out_perm, weights, inv, T, K, residual=res).reshape(shape)
-        if self.ep_size == 1 and st["w4"] and x2d.dtype == torch.bfloat16 and self._w4_tile(st, T * K):
-            # prefill: both projections on the tensor-core tile kernel, which gathers the rows itself
+        if self.ep_size == 1 and st["w4"] and x2d.dtype == torch.bfloat16 and self._w4_tile(st, T * K, xp_tok is None):
+            # prefill: the tensor-core tile kernel, which gathers the rows itself
             status = self._status_word(x2d.device)
             h = run("grouped_swiglu", w4a16_grouped_swiglu_gather, x2d, perm, K, st["gate_proj"], st["up_proj"], off32,
                     st["group_size"], status=status)
@@ -475,15 +475,14 @@ class Qwen3MoEBlock(nn.Module):
         h = run("grouped_swiglu", moe_grouped_swiglu, rows, st["w13"], off32, zero_init=False, status=status)
         return run("grouped_down", moe_grouped_gemm, h, st["w2"], off32, zero_init=False, out=out, status=status)
 
-    def _w4_tile(self, st, slots: int) -> bool:
-        """Whether both projections run on the tensor-core tile kernel: more than eight slots per expert on average
-        (the rule of the library's own dispatch) and tensors it covers."""
-        if self.w4_kernel != "stream" or slots <= 8 * self.num_local_experts:
-            return False
-        if any(st[p][2].data_ptr() % 16 for p in ("gate_proj", "up_proj")):
+    def _w4_tile(self, st, slots: int, prepare: bool = True) -> bool:
+        """Whether the gate/up projection runs on the tensor-core tile kernel: by the rule of the library's own dispatch
+        (``prepare``: the stream kernel's activations are yet to be prepared), and tensors the kernel takes."""
+        if self.w4_kernel != "stream" or any(st[p][2].data_ptr() % 16 for p in ("gate_proj", "up_proj")):
             return False
         qw = st["gate_proj"][0]
-        return w4a16_gather_supported(qw.shape[1] * 8, qw.shape[2], st["group_size"], self.num_local_experts)
+        return bool(_cabi.load().mq_w4a16_tile_pays(slots, self.num_local_experts, qw.shape[2], qw.shape[1] * 8,
+                                                    st["group_size"], 1, int(prepare)))
 
     def _w4_stream(self, st) -> bool:
         """Whether the prepared-activation path applies (``w4_kernel == "stream"`` and the shapes are covered)."""

@@ -22,6 +22,13 @@ def kperm_index(n):
     return (c & ~7) | (((c & 3) << 1) | ((c >> 2) & 1))
 
 
+def off_grid(t):
+    """The same values four bytes off the 16-byte grid."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:] = t.reshape(-1)
+    return flat[1:].view(t.shape)
+
+
 def dev_set(p):
     return tuple(t.to(DEV) for t in (p.qweight, p.scales.to(torch.bfloat16), p.qzeros))
 
@@ -103,7 +110,9 @@ def test_stream_kernel_gate_up_and_down_match_the_oracle(T, H, E, K, I, skew):
         "natural order": w4a16_stream_gemm(h, None, *down, off32, x_shuffled=False, status=status),
         "shuffled": w4a16_stream_gemm(h_shuf, None, *down, off32, status=status),
         "shuffled, sums given": w4a16_stream_gemm(h_shuf, hs, *down, off32, status=status),
-        "cp.async kernel": w4a16_grouped_gemm(h, *down, off32, zero_init=False),
+        "as dispatched": w4a16_grouped_gemm(h, *down, off32, zero_init=False),
+        # at these sizes the dispatch prefers the tile kernel, which wants zero points on the 16-byte grid
+        "cp.async kernel": w4a16_grouped_gemm(h, *down[:2], off_grid(down[2]), off32, zero_init=False),
     }.items():
         try:
             cases.w4_output_bar(o.cpu(), o32, o64)

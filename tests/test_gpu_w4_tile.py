@@ -1,7 +1,8 @@
 """The W4A16 tile kernel for prefill-size groups (csrc/w4a16_tile.cu): single linears and grouped projections at the
 edges of its tiles (rows 9 to 129 around the 16-row steps and the 128-row tile, columns that end inside a tile or after
 the first of a pair, one and several quantisation groups, empty experts), with contiguous and with gathered rows, and
-with several tiles to a CTA.
+with several tiles to a CTA.  Where a call has too few rows for the kernel to pay, the dispatch sends it elsewhere: groups of
+few rows are tested beside large ones.
 
 Single linears are held to the fp32 result of the oracle's formula: the kernel multiplies exact integers q - z and adds
 fp32 sums, so only the summation order (about 2^-22 of the sum of magnitudes) and the final rounding to bf16 (2^-9
@@ -65,15 +66,35 @@ def test_grouped_projections_match_the_oracle(T, H, E, K, I, hot):
     rows = gather_rows(xd, perm, K)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     h = w4a16_grouped_swiglu_gather(xd, perm, K, dev_set(gate), dev_set(up), off32, status=status)
-    assert torch.equal(w4a16_grouped_swiglu(rows, dev_set(gate), dev_set(up), off32), h)
+    plain = w4a16_grouped_swiglu(rows, dev_set(gate), dev_set(up), off32)
+    if _cabi.load().mq_w4a16_tile_pays(T * K, E, I, H, 128, 1, 0):
+        assert torch.equal(plain, h)
     off, sets = off32.cpu(), tuple((p.qweight, p.scales.to(torch.bfloat16), p.qzeros) for p in (gate, up))
     h32, h64 = (cases.w4_grouped_reference(rows.cpu(), sets, off, t) for t in (torch.float32, torch.float64))
     cases.w4_output_bar(h.cpu(), h32, h64)
+    cases.w4_output_bar(plain.cpu(), h32, h64)
     if down is not None:
         o = w4a16_grouped_gemm(h, *dev_set(down), off32)
         dset = ((down.qweight, down.scales.to(torch.bfloat16), down.qzeros),)
         o32, o64 = (cases.w4_grouped_reference(h.cpu(), dset, off, t) for t in (torch.float32, torch.float64))
         cases.w4_output_bar(o.cpu(), o32, o64)
+    assert status.item() == 0
+
+
+@pytest.mark.parametrize("N,K", [(32, 128), (128, 256), (96, 384), (160, 128)])
+def test_plain_projection_of_small_groups_beside_a_large_one(N, K):
+    g = torch.Generator().manual_seed(N + K)
+    counts = [9, 16, 0, 17, 1, 15, 1200]
+    off = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32)
+    S, E = int(off[-1]), len(counts)
+    assert _cabi.load().mq_w4a16_tile_pays(S, E, N, K, 128, 0, 0)
+    p = synthetic._w4_proj(g, E, K, N, 128)
+    x = torch.randn(S, K, generator=g).to(torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = w4a16_grouped_gemm(x.to(DEV), *dev_set(p), off.to(DEV), status=status).cpu()
+    sets = ((p.qweight, p.scales.to(torch.bfloat16), p.qzeros),)
+    r32, r64 = (cases.w4_grouped_reference(x, sets, off, t) for t in (torch.float32, torch.float64))
+    cases.w4_output_bar(got, r32, r64)
     assert status.item() == 0
 
 
@@ -115,10 +136,18 @@ def test_swiglu_keeps_the_exact_quotient_where_the_stream_kernel_did_not_run(cou
     S = int(off[-1])
     assert S > 8 * len(counts)
     x = (torch.randn(S, H, generator=g) * 0.3).to(torch.bfloat16).to(DEV)
-    want = torch.nn.functional.silu(w4a16_grouped_gemm(x, *gate, off)) * w4a16_grouped_gemm(x, *up, off)
-    assert torch.equal(w4a16_grouped_swiglu(x, gate, up, off), want)
+    # the projections by themselves, in the same order of the sums: each group's rows forty times over, so that the plain
+    # call pays on the tile kernel, which keeps the rows of a group apart
+    many = torch.cat([x[s:t].repeat(40, 1) for s, t in zip(off.tolist(), off.tolist()[1:])])
+    first = torch.cat([40 * s + torch.arange(t - s) for s, t in zip(off.tolist(), off.tolist()[1:])]).to(DEV)
+    gate_rows, up_rows = (w4a16_grouped_gemm(many, *w, off * 40)[first] for w in (gate, up))
+    want = torch.nn.functional.silu(gate_rows) * up_rows
     perm = torch.arange(S, dtype=torch.int32, device=DEV)
     assert torch.equal(w4a16_grouped_swiglu_gather(x, perm, 1, gate, up, off), want)
+    direct = w4a16_grouped_swiglu(x, gate, up, off)
+    if E == 3:                     # goes to the cp.async kernel, as its projections do
+        want = torch.nn.functional.silu(w4a16_grouped_gemm(x, *gate, off)) * w4a16_grouped_gemm(x, *up, off)
+    assert torch.equal(direct, want)
 
 
 def test_gather_entry_point_rejects_what_the_kernel_does_not_cover():

@@ -362,3 +362,31 @@ def test_expert_parallel_w4a16_calls_say_how_many_rows_are_a_ranks_own(monkeypat
     seen.clear()
     blk._forward_peer(x, st, None, None, None, None, off, T, K, E)
     assert seen == [(G * T * K, T * K)] * 2
+
+
+def test_which_kernel_a_w4a16_call_goes_to():
+    """The rule by sizes at the places where both sides were measured (us, streaming kernels | tile kernel)."""
+    pays = _cabi.load().mq_w4a16_tile_pays
+
+    def fused(S, E, N, K, prepare=1):
+        return pays(S, E, N, K, 128, 1, prepare)
+
+    def one(S, E, N, K):
+        return pays(S, E, N, K, 128, 0, 0)
+    for tile, calls in ((0, [(232, 16, 128, 2048), (254, 8, 128, 1792), (116, 8, 256, 1536), (448, 16, 128, 2048),
+                             (64, 1, 768, 2048), (100, 2, 384, 1024), (1024, 128, 768, 2048)]),   # 12|21 12|19 11|18 15|21 11|20 9|13
+                        (1, [(1280, 128, 768, 2048), (2048, 128, 768, 2048), (32768, 128, 768, 2048), (160, 16, 768, 512),
+                             (400, 16, 384, 1024), (520, 64, 384, 1024), (3000, 8, 768, 2048)])):  # 109|103 152|104 - 19|10 20|14
+        for c in calls:
+            assert fused(*c) == tile, c
+    for tile, calls in ((0, [(9, 1, 512, 512), (16, 1, 4096, 512), (16, 1, 2048, 2048), (27, 3, 1024, 384),
+                             (152, 16, 1280, 128), (1160, 128, 1536, 128), (1104, 128, 768, 256)]),
+                        (1, [(17, 1, 512, 512), (17, 1, 2048, 4096), (33, 1, 512, 2048), (500, 1, 2048, 4096),
+                             (160, 16, 2048, 768), (1280, 128, 2048, 768), (32768, 128, 2048, 768)])):
+        for c in calls:
+            assert one(*c) == tile, c
+    assert fused(64, 16, 768, 2048) == 0 and one(64, 16, 2048, 768) == 0          # four rows a group: never
+    # more groups than the stream kernel takes: the cp.async kernel is the alternative
+    assert fused(8 * 400 + 1, 400, 768, 2048) == 1 and fused(8 * 400, 400, 768, 2048) == 0
+    # sizes that the tile kernel does not take, and nonsense
+    assert pays(4000, 4, 768, 2048, 64, 1, 0) == 0 and one(4000, 4, 100, 2048) == 0 and one(-1, 0, 0, 0) == 0
