@@ -619,10 +619,19 @@ bool pair_map_gate_up(CUtensorMap* map, const void* base, int64_t experts, int64
 // of a short K with every expert hit stays with the single-CTA kernel: a tile is then 12 stages, too few to hide the
 // two epilogues of a pair behind (K = 768, N = 2048, 128 experts, us, single against pair: 95 | 101 at 144 rows per
 // expert, 111 | 118 at 256, 131 | 136 at 272; but 48 | 44 with 50 of the experts hit by one row, where the finer tiles
-// spread better).  SwiGLU over K = 2048, gathered: 94 | 73 with 50 rows, 176 | 148 at 48 per expert, 222 | 208 at 256,
-// 281 | 230 at 272, 355 | 327 at 512.
+// spread better).  From K = 1024 on it goes by pairs up to 100 rows a group (K 2048, N 768, 128 experts: 85 | 81 at 92 rows;
+// with fewer 8 to 28 % faster on average over 140 shapes), and with more where there are few groups and a long K (16 and 32
+// groups: 0.86 to 1.39 times as fast); 64 and more groups are slower (89 | 98 at 122 rows, 100 | 110 at 191), as is K 1024 (16
+// groups, N 1536: 20.0 | 22.9 at 215 rows).  SwiGLU over K = 2048, gathered: 94 | 73 with 50 rows, 176 | 148 at 48 per expert, 222 | 208 at 256,
+// 281 | 230 at 272, 355 | 327 at 512.  Two ranges of it stay there as well.  Fewer than 16 groups of over 256 rows: a pair's
+// tile is four times a CTA's, and a round that is not full costs as much more (8 experts: 31 | 50 at 2217 rows, K 2048,
+// N 256; 28 | 42 at 622, K 1792, N 768; by 5 % the slower on average over 36 shapes).  A K of 512 or less with up to 32 groups of 128 rows or
+// more: again too few stages (K 512, N 768, 16 experts: 16.0 | 16.8 at 144 rows, 25.3 | 29.7 at 512; 32 experts: 27.8 | 29.3
+// at 200; but 69 | 61 with 128 experts, 144 rows, and 14.4 | 10.1 with N 128, 16 experts).  Of 871 measured calls (8 to 128 experts, K 512 to 2048, even
+// and skewed) the pair kernel is then the slower one by over 3 % in 27, the faster one by 22 % on average.
 bool grouped_gemm_pair_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, bool swiglu) {
-  if (!swiglu && Kd < 1024 && S > E) return false;
+  if (!swiglu && ((Kd < 1024 && S > E) || (S > 100 * E && (E >= 64 || Kd < 1280)))) return false;
+  if (swiglu && ((E < 16 && S > 256 * E) || (Kd <= 512 && E <= 32 && N > 128 && S >= 128 * E))) return false;
   return Kd % 128 == 0 && N % (swiglu ? 128 : 256) == 0 && E <= P_MAX_E && S < ((int64_t)1 << 30) &&
          period * N * 2 < ((int64_t)1 << 31) && (S / 256 + 2 * E) * (N / 128) < ((int64_t)1 << 30);
 }
