@@ -12,7 +12,7 @@
 namespace mq {
 
 bool tc5_covers(int64_t S, int64_t E, int64_t N, int64_t Kd, bool swiglu);
-bool generic_small_groups(int64_t S, int64_t E, int64_t N);
+bool generic_small_groups(int64_t S, int64_t E, int64_t N, bool swiglu);
 int grouped_gemm_generic_dispatch(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E,
                                   int64_t period, int64_t N, int64_t Kd, int dtype, bool swiglu, void* out,
                                   cudaStream_t st, const int32_t* perm, int64_t top_k);
@@ -43,7 +43,7 @@ BlockPlan plan_of(const mq_moe_layer& L, int64_t T) {
     p.gather_in_kernel = p.tile || p.stream;
   } else {
     p.tc5 = L.dtype == MQ_BF16 && tc5_covers(S, E, I, H, true) && T * H < ((int64_t)1 << 32);
-    p.gather_in_kernel = p.tc5 || generic_small_groups(S, E, I);
+    p.gather_in_kernel = p.tc5 || generic_small_groups(S, E, I, true);
   }
   return p;
 }

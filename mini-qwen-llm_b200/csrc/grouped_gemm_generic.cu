@@ -143,7 +143,7 @@ grouped_gemm_generic(const T* __restrict__ a, const T* __restrict__ w, const int
   }
 }
 
-// Groups of few rows (an average of at most 32): tiles of 16 rows x 32 columns, so that a small layer spreads over the
+// Groups of few rows (generic_small_groups): tiles of 16 rows x 32 columns, so that a small layer spreads over the
 // whole GPU, and 128 k at a time through registers into shared memory, the next 128 already on their way.  A layer of
 // these sizes is bound by the latency of its K loop: with the 64 x 64 tiles above and 16 k per round trip the two
 // projections of an fp32 layer of 64 tokens (8 experts, 256 x 512) took 23.5 and 33.6 us.
@@ -301,14 +301,20 @@ int launch_generic(const void* a, const void* w, const int32_t* offsets, int64_t
 }  // namespace
 
 // Whether the small-group kernel takes these sizes: at most 32 rows per group on average (more rows fill the 64-row
-// tiles well enough to need a quarter of the weight reads).
-bool generic_small_groups(int64_t S, int64_t E, int64_t N) { return S <= 32 * E && (N + GS_TN - 1) / GS_TN <= 65535; }
+// tiles well enough to need a quarter of the weight reads), and fewer where there are groups enough for the 64-row tiles
+// to fill the GPU.  us, 64-row | 16-row tiles, fp32, K 256, N 512.  Plain: 32 groups of 32 rows 35.6 | 27.6; 64 of 24
+// 48.5 | 40.3, of 28 42.0 | 43.9; 128 of 24 86 | 84, of 32 86 | 101; 256 of 16 142 | 138, of 20 143 | 161.  Fused: 32 of 32
+// 52.4 | 45.3; 64 of 28 98 | 73; 96 of 28 104 | 110; 128 of 32 150 | 163; 256 of 20 254 | 247, of 24 255 | 280.
+bool generic_small_groups(int64_t S, int64_t E, int64_t N, bool swiglu) {
+  const bool few = S <= 1024 || (swiglu ? S <= 28 * E && S <= 5120 : S <= 24 * E && S <= 4096);
+  return S <= 32 * E && few && (N + GS_TN - 1) / GS_TN <= 65535;
+}
 
 // perm (small groups only): row p is a[perm[p] / top_k].
 int grouped_gemm_generic_dispatch(const void* a, const void* w, const int32_t* offsets, int64_t S, int64_t E,
                                   int64_t period, int64_t N, int64_t Kd, int dtype, bool swiglu, void* out,
                                   cudaStream_t st, const int32_t* perm, int64_t top_k) {
-  if (generic_small_groups(S, E, N)) {
+  if (generic_small_groups(S, E, N, swiglu)) {
     if (dtype == MQ_F32) return launch_small<float>(a, perm, top_k, w, offsets, S, E, period, N, Kd, swiglu, out, st);
     if (dtype == MQ_BF16)
       return launch_small<__nv_bfloat16>(a, perm, top_k, w, offsets, S, E, period, N, Kd, swiglu, out, st);

@@ -12,7 +12,9 @@ DEV = torch.device("cuda", 0)
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,N,Kd", [((1, 0, 15), 31, 4), ((16, 17, 1), 32, 127), ((32, 3, 0), 33, 128),
-                                       ((7, 31, 2), 96, 260), ((20, 20, 20), 5, 129)])
+                                       ((7, 31, 2), 96, 260), ((20, 20, 20), 5, 129),
+                                       # many groups: the fused call here, the plain one with 64-row tiles; then both so
+                                       ((26,) * 128, 33, 20), ((30,) * 128, 33, 20)])
 def test_small_groups(dtype, rows, N, Kd):
     if dtype != torch.float32 and Kd % 64 == 0 and N % 128 == 0:
         pytest.skip("the tcgen05 kernel takes this shape")
