@@ -89,5 +89,8 @@ def test_pair_shared_weights_and_partial_offsets(counts):
     for out in (plain, h):
         assert not out[:lo].any() and not out[hi:].any()
     close(plain[lo:hi], plain_ref[lo:hi])
-    close(h[lo:hi], ref[lo:hi])
+    # gate, silu, up and their product may each fall one bf16 step apart (2^-7 of the value); below zero, where |silu'| is up
+    # to 0.1, a step of the gate (2^-5 for |g| < 8) moves the product by 0.1 * 2^-5 * |u|, |u| < 8
+    torch.testing.assert_close(h[lo:hi].cpu().float(), ref[lo:hi].float(), rtol=2 ** -5, atol=2.5e-2)
+    assert (h[lo:hi].cpu() != ref[lo:hi]).float().mean() < 0.01
     assert torch.equal(gathered[lo:hi], h[lo:hi])
