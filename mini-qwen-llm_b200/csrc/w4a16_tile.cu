@@ -560,7 +560,8 @@ bool w4a16_tile_faster(int64_t rows, int64_t E, int64_t N, int64_t Kd, bool swig
   const double blocks = ceil(E == 1 ? per_group : per_group + 0.55);       // of eight rows, in the larger groups
   if (swiglu) {
     const double tile = 3.0 + rounds * (0.55 * units + 2.0);
-    if (rows < 32 && alternative == 0) return tile < 2.3 + blocks * (1.7 + 0.0019 * k);
+    if (rows < 32 && alternative == 0)           // the cp.async kernel, and an exact SwiGLU, which takes 1.5 us longer
+      return tile + 1.5 < 2.3 + blocks * (1.7 + 0.0019 * k);
     // the stream kernel: items of eight rows x `panels` of 32 columns, dealt out to all SMs
     const int panels = w4a16_stream_panels(rows, E, N, true);
     const double items = (E == 1 ? ceil(per_group) : (per_group + 0.6) * E) * (double)((N / 32 + panels - 1) / panels);
@@ -570,7 +571,7 @@ bool w4a16_tile_faster(int64_t rows, int64_t E, int64_t N, int64_t Kd, bool swig
   }
   const double tile = 2.7 + rounds * (0.5 * units + 2.0), words = (double)N * k * E;
   if (rows <= 32)                                // the cp.async kernel with K split over four warps
-    return tile < 2.3 + blocks * (1.1 + 0.0017 * k) + words / 7e6;
+    return tile < 2.3 + blocks * (1.1 + 0.0017 * k) + (E == 1 ? words / 7e6 : 0.0);
   // and without: a warp takes a group's blocks of eight rows one after the other
   const double even = 5.7 + 0.0025 * k + (per_group + 0.4) * words / 4.5e6, chain = 4.0 + (per_group + 0.5) * 0.006 * k;
   return tile < (even > chain ? even : chain);
