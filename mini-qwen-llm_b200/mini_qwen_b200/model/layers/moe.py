@@ -116,7 +116,8 @@ class Qwen3MoEBlock(nn.Module):
         # gathers through a slot table; "slots": one copy per slot (W4A16 experts, more than 8 ranks)
         self.ep_dispatch = "unique"
         # W4A16 experts: "stream" = activations prepared once (rows gathered in the k order the MMA wants, group
-        # sums), gate/up on the TMA-staged stream kernel, down on the cp.async kernel (the default);
+        # sums), gate/up on the TMA-staged stream kernel, down on the cp.async kernel, and either on the tensor-core tile
+        # kernel at the sizes where that is the faster one (the default);
         # "mma" = both projections on the cp.async kernel from materialised rows; "tc" = the tcgen05 kernel
         # with the weights dequantised into tensor memory; "auto" = "tc" by the number of slots per expert
         self.w4_kernel = "stream"
