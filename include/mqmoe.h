@@ -256,12 +256,13 @@ int mq_w4a16_grouped_gemm(const void* x, const int32_t* qweight, const void* sca
                           int64_t S, int64_t E, int64_t weight_period, int64_t N, int64_t Kd, int64_t group_size,
                           void* out, void* stream);
 
-/* Fused W4A16 gate/up projection with SwiGLU (bf16 rounding after gate, silu, up and the
- * product, as LinearW4A16 returns bf16).  Both projections share shapes: Kd = H, N = I. */
 /* One linear (LinearW4A16.forward, mini_qwen/model/layers/linear_w4a16.py:31-36): mq_w4a16_grouped_gemm with a single
  * group of M rows, without an offsets array. */
 int mq_w4a16_linear(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros, int64_t M,
                     int64_t N, int64_t Kd, int64_t group_size, void* out, void* stream);
+
+/* Fused W4A16 gate/up projection with SwiGLU (bf16 rounding after gate, silu, up and the
+ * product, as LinearW4A16 returns bf16).  Both projections share shapes: Kd = H, N = I. */
 int mq_w4a16_grouped_swiglu(const void* x,
                             const int32_t* qweight_gate, const void* scales_gate, const int32_t* qzeros_gate,
                             const int32_t* qweight_up, const void* scales_up, const int32_t* qzeros_up,

@@ -156,17 +156,12 @@ grouped_prepare(const void* __restrict__ offsets, int E, int64_t S, int64_t row_
     if (status != nullptr && threadIdx.x == 0) *status = 0;
   }
   if (out == nullptr) return;
-  // a row between the first and the last offset lies in some group
+  // Offsets ascend: the rows between the first and the last of them are the covered ones.
   const int64_t lo = off(0), hi = off(E);
   if (lo <= 0 && hi >= S) return;
   const int lane = threadIdx.x & 31;
   for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < S; r += (int64_t)gridDim.x * 8) {
-    bool covered = r >= lo && r < hi;
-    if (!covered) {
-      for (int e = lane; e < E; e += 32) covered = covered || (off(e) <= r && r < off(e + 1));
-      covered = __any_sync(0xffffffffu, covered);
-    }
-    if (covered) continue;
+    if (r >= lo && r < hi) continue;
     uint8_t* o = out + r * row_bytes;
     if (vec) {
       for (int64_t i = lane; i < row_bytes / 16; i += 32) reinterpret_cast<uint4*>(o)[i] = make_uint4(0, 0, 0, 0);
