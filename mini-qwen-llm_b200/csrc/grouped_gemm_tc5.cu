@@ -27,8 +27,6 @@
 //
 // Every mbarrier wait is bounded: when it runs out the kernel sets MQ_DEV_WAIT_EXPIRED in the status
 // word, all roles leave their loops, and TMEM is freed before the CTA exits.
-#include <mutex>
-
 #include "tc5.cuh"
 
 namespace mq {
@@ -592,26 +590,9 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
 }
 
 // ---------------------------------------------------------------------------------------------- host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
 // 2-D bf16 row-major [rows, cols] tensor, box = 64 columns x box_rows rows, 128-byte swizzle.
 bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * 2};
@@ -621,17 +602,6 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, 
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
-}
-
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
 }
 
 }  // namespace
@@ -666,7 +636,7 @@ int grouped_gemm_tc5(const void* a, const void* w, const int32_t* offsets, int64
   const int64_t tiles_max = ((S + TN_MAX - 1) / TN_MAX + E) * nwt;
   // gathering: the number of slots is offsets[E], known only on the device (it is not T * top_k when the
   // rows are a receive buffer addressed through a slot table), so the grid is not trimmed
-  const int grid = (int)(!gather && tiles_max < sm_count() ? tiles_max : sm_count());
+  const int grid = (int)(!gather && tiles_max < device_sm_count() ? tiles_max : device_sm_count());
   const __nv_bfloat16* xa = reinterpret_cast<const __nv_bfloat16*>(a);
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
   // the attribute is per device; setting it is cheap, so it is set on every call

@@ -8,11 +8,7 @@
 // chunking, in the same order, as the mma.sync kernel in router.cu, which this kernel replaces for
 // batches of 256 tokens and more.  Two TMEM accumulators alternate, so the fold of one chunk runs
 // under the MMAs of the next.  All waits are bounded.
-#include <cuda.h>
-
-#include <mutex>
-
-#include "common.cuh"
+#include "tc5.cuh"
 
 namespace mq {
 namespace {
@@ -243,23 +239,8 @@ router_logits_tc5_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   }
 }
 
-typedef CUresult (*RtEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-RtEncodeFn rt_encode_fn() {
-  static RtEncodeFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<RtEncodeFn>(p);
-  });
-  return fn;
-}
 bool rt_map(CUtensorMap* map, bool bf16, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  RtEncodeFn fn = rt_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * 2};

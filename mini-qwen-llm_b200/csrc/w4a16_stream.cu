@@ -39,11 +39,7 @@
 //     the other warps' partials are certain to be there: no warp ever stands at a barrier for them.
 //
 // Every mbarrier wait is bounded; on expiry MQ_DEV_WAIT_EXPIRED is set and all warps leave their loops.
-#include <cuda.h>
-
-#include <mutex>
-
-#include "common.cuh"
+#include "tc5.cuh"
 
 namespace mq {
 namespace {
@@ -650,30 +646,13 @@ w4a16_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------------- host
-typedef CUresult (*WsEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-WsEncodeTiledFn ws_encode_fn() {
-  static WsEncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<WsEncodeTiledFn>(p);
-  });
-  return fn;
-}
-
 // qweight [period, Kd/8, N] int32 seen as (32 columns, Kd/8 word rows, N/32 panels, period); a box is
 // (32, box_rows, box_panels, 1) and lands as box_panels dense panels of box_rows 128-byte rows, the 16-byte
 // pieces of a row exchanged by the 128-byte swizzle (piece c of row r sits at position c ^ (r & 7)).  Word rows
 // and panels outside the tensor read as zero.
 bool ws_make_map(CUtensorMap* map, const void* qweight, int64_t period, int64_t Kd, int64_t N, int box_rows,
                  int box_panels) {
-  WsEncodeTiledFn fn = ws_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
   cuuint64_t dims[4] = {32, (cuuint64_t)(Kd / 8), (cuuint64_t)(N / 32), (cuuint64_t)period};
   cuuint64_t strides[3] = {(cuuint64_t)N * 4, 128, (cuuint64_t)(Kd / 8) * (cuuint64_t)N * 4};
@@ -705,17 +684,6 @@ int ws_dynamic_smem_bytes(const void* kernel) {
   return room;
 }
 
-int ws_sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace
 
 bool w4a16_stream_covers(int64_t S, int64_t E, int64_t period, int64_t N, int64_t Kd, int64_t group) {
@@ -734,7 +702,7 @@ int w4a16_stream_panels(int64_t S, int64_t E, int64_t N, bool swiglu) {
     if (swiglu && c >= 8) continue;                 // a gate + up stage of 8 panels would not fit the ring
     const int64_t items = active * ((panels + c - 1) / c);
     // 16 panels = no K split at all (no partial sums to add up): worth fewer items per SM
-    if (items >= (c == 16 ? 3 : 4) * ws_sm_count()) return c;
+    if (items >= (c == 16 ? 3 : 4) * device_sm_count()) return c;
   }
   return 1;
 }
@@ -795,7 +763,7 @@ int w4a16_stream(const void* x, const float* xs, int x_format, const int32_t* pe
   CUtensorMap map0, map1;
   if (!ws_make_map(&map0, qw0, period, Kd, N, RS, CW) || !ws_make_map(&map1, swiglu ? qw1 : qw0, period, Kd, N, RS, CW))
     return MQ_ERR_DRIVER_ENTRY;
-  const int grid = ws_sm_count();
+  const int grid = device_sm_count();
   const bool xsum = xs != nullptr;
 #define MQ_WS_LAUNCH(SW, XSH, XSU, F16)                                                                            \
   do {                                                                                                             \

@@ -30,11 +30,7 @@
 // 1000 cycles per quantisation group and tile (the dequantisation warps need the same 1000, the fold
 // warps 450, and they overlap); rotating the k steps over independent accumulators changes nothing.
 // The shape pays off only with more tokens per expert than a decode batch has.
-#include <cuda.h>
-
-#include <mutex>
-
-#include "common.cuh"
+#include "tc5.cuh"
 #include "w4_prep.cuh"
 
 namespace mq {
@@ -486,26 +482,9 @@ w4_prep_rows(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pe
   }
 }
 
-typedef CUresult (*W4EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-W4EncodeFn w4_encode_fn() {
-  static W4EncodeFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<W4EncodeFn>(p);
-  });
-  return fn;
-}
-
 bool w4_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const void* base, uint64_t rows,
                uint64_t cols, uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle sw) {
-  W4EncodeFn fn = w4_encode_fn();
+  EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * (uint64_t)elem_bytes};
@@ -513,17 +492,6 @@ bool w4_map_2d(CUtensorMap* map, CUtensorMapDataType dt, int elem_bytes, const v
   cuuint32_t estr[2] = {1u, 1u};
   return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-int w4_sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
 }
 
 bool w4_tc_covers(int64_t S, int64_t Ew, int64_t N, int64_t Kd, int64_t group_size) {
@@ -570,7 +538,7 @@ static int w4_tc_launch(bool swiglu, const void* xp, const float* xs, const int3
     return MQ_ERR_DRIVER_ENTRY;
   const int64_t nwt = N / W_TM;
   const int64_t tiles_max = ((S + W_TN - 1) / W_TN + E) * nwt;
-  const int grid = (int)(tiles_max < w4_sm_count() ? tiles_max : w4_sm_count());
+  const int grid = (int)(tiles_max < device_sm_count() ? tiles_max : device_sm_count());
   W4TcProj p0{reinterpret_cast<const __nv_bfloat16*>(sc0), qz0};
   W4TcProj p1{reinterpret_cast<const __nv_bfloat16*>(swiglu ? sc1 : sc0), swiglu ? qz1 : qz0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
