@@ -492,38 +492,23 @@ route_tokens_kernel(const void* __restrict__ xv_, int xdt, const void* __restric
     const int e0 = eg * 32 + warp;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (F32) {
-      // Every piece's eight products are added up by themselves and the pieces' sums in pairs, as deep a tree as the
-      // expert-major kernel's (eight products a thread, then the threads): one chain of H / 32 products a lane would
-      // add up fp32 logits less exactly.
-      for (int p0 = 0; p0 < pieces; p0 += 32 * MAXP) {
-        float part[MAXP][4];
+      // Every piece's eight products are added up by themselves, then the pieces' sums one after the other, as the
+      // expert-major kernel adds a thread's eight products and then the warps' sums: one chain of H / 32 products a lane
+      // would add up fp32 logits less exactly.
+      for (int pc = lane; pc < pieces; pc += 32) {
+        float a[8], b[4][8];
+        load8(xv_, xdt, (size_t)t * H + 8 * pc, a);
 #pragma unroll
-        for (int i = 0; i < MAXP; ++i) {
-          const int pc = p0 + lane + 32 * i;
+        for (int j = 0; j < 4; ++j)
+          if (e0 + 8 * j < E) load8(wv_, wdt, (size_t)(e0 + 8 * j) * H + 8 * pc, b[j]);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
-          if (pc < pieces) {
-            float a[8], b[4][8];
-            load8(xv_, xdt, (size_t)t * H + 8 * pc, a);
+        for (int j = 0; j < 4; ++j)
+          if (e0 + 8 * j < E) {
+            float part = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (e0 + 8 * j < E) load8(wv_, wdt, (size_t)(e0 + 8 * j) * H + 8 * pc, b[j]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (e0 + 8 * j < E) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) part[i][j] = fmaf(a[q], b[j][q], part[i][j]);
-              }
+            for (int q = 0; q < 8; ++q) part = fmaf(a[q], b[j][q], part);
+            acc[j] += part;
           }
-        }
-#pragma unroll
-        for (int d = 1; d < MAXP; d *= 2)
-#pragma unroll
-          for (int i = 0; i < MAXP; i += 2 * d)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) part[i][j] += part[i + d][j];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] += part[0][j];
       }
     } else {
       const uint16_t* xr = reinterpret_cast<const uint16_t*>(xv_) + (size_t)t * H;
