@@ -546,7 +546,7 @@ TileShape tile_shape(int64_t rows, int64_t E, int64_t N, bool swiglu, int sms) {
 // compared by their times in us.  The figures are fits to 960 calls of 1 to 128 groups of over 8 to 100 rows (K and N 128
 // to 4096, even and skewed).  Fused, as a block calls it: the slower kernel is chosen by more than 4 % for 6 of 261, by
 // 15 % at most; by the eight rows alone for 32, up to 1.75 times as long (16 groups of 14 rows, K 2048, N 128: 12.2 us on
-// the stream kernel, 21.4 on this; one group of 32 rows, N 768: 7.5 | 20.1).  Plain: for 23 of 697, most of them of K 128,
+// the stream kernel, 21.4 on this; one group of 32 rows, N 768: 7.5 | 20.1).  Plain: for 20 of 697, most of them of K 128,
 // where skewed groups, which a rule on sizes does not see, make the cp.async kernel up to 3.6 times slower.
 // alternative: the fused projection's other kernel: 0 stream or (under 32 rows) cp.async, as the dispatch has it; 1 stream
 // on activations that are prepared already; 2 stream after a launch that prepares them.
